@@ -113,9 +113,7 @@ __device__ __forceinline__ CellParams pheno_params(int ph, float gks_s, float gk
 
 // Stimulus current of a cell of variant var at step istep: the sum of the
 // amplitudes of its sites that fire then (each variant has its own sites).
-__device__ __forceinline__ float stim_current(const MonoArgs& a, uint32_t bits, int64_t istep,
-                                              int var) {
-  uint32_t on = bits & (uint32_t)a.site_on[var * a.site_stride + istep];
+__device__ __forceinline__ float site_current(const MonoArgs& a, uint32_t on, int var) {
   float I = 0.0f;
   while (on) {
     int s = __ffs(on) - 1;
@@ -123,6 +121,10 @@ __device__ __forceinline__ float stim_current(const MonoArgs& a, uint32_t bits, 
     on &= on - 1;
   }
   return I;
+}
+__device__ __forceinline__ float stim_current(const MonoArgs& a, uint32_t bits, int64_t istep,
+                                              int var) {
+  return site_current(a, bits & (uint32_t)a.site_on[var * a.site_stride + istep], var);
 }
 
 // One threshold crossing between snapshots (t0, v0) -> (t1, v1), linear
@@ -1197,6 +1199,10 @@ __global__ void cn_cond_kernel(cudaGraphConditionalHandle hd, CnArgs c, int init
   cudaGraphSetConditional(hd, (!c.iscal[CI_DONE] && n < c.max_iter) ? 1u : 0u);
 }
 
+}  // namespace hp
+#include "mono_resident.cuh"
+namespace hp {
+
 // Host: halo copy table of the pipelined and split-diffusion kernels for
 // one brick shape: the union of the tile elements the stencil reads, minus
 // the brick's own voxels (the 7-point operator reads face neighbours only,
@@ -1274,6 +1280,7 @@ typedef void (*CnFn)(MonoArgs, CnArgs);
 typedef void (*CnPassFn)(MonoArgs, CnArgs);
 typedef void (*PipeFn)(MonoArgs, int);  // also the diffusion half of the split step
 typedef std::vector<uint32_t> (*HaloFn)(bool);
+typedef void (*ResFn)(MonoArgs, CnArgs, ResArgs, int);
 
 struct ShapeEntry {
   int bi, bj, bk;
@@ -1319,6 +1326,10 @@ struct HpMono {
   CnFn cn;           // theta > 0: set-up pass (Jacobi diagonal), or null
   CnPassFn cn_start, cn_apply;  // tiled passes: start of a solve, A p
   CnArgs cn_a;
+  ResFn res;            // resident steps (hearts that fit at one cell per thread), or null
+  ResArgs res_a;
+  int res_grid, res_threads;
+  size_t res_smem;
   int cn_grid;       // persistent grid of the set-up pass
   int cn_pgrid;      // persistent grid of the tiled passes
   int cn_vgrid;      // grid of the vector kernels
@@ -1524,9 +1535,7 @@ static hp_status setup_cn(HpMono* h, const ShapeEntry* se, const HpMonoDesc* d, 
   HP_CUDA_TRY(cudaMemsetAsync(c.ticket, 0, sizeof(unsigned int), s));
   // padding entries of the CG vectors stay zero (the passes skip them)
   for (float* v : {c.x, c.r, c.p, c.q}) HP_CUDA_TRY(cudaMemsetAsync(v, 0, n * sizeof(float), s));
-  HP_CUDA_TRY(cudaMallocHost((void**)&h->cn_host, 2 * sizeof(int32_t)));
   h->a.cn_x = c.x;
-  HP_CUDA_TRY(cudaStreamCreateWithFlags(&h->cn_body_stream, cudaStreamNonBlocking));
   h->cn<<<h->cn_grid, h->bv, 0, s>>>(h->a, c);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
@@ -1638,6 +1647,95 @@ static hp_status cn_build_graph(HpMono* h, int n, cudaStream_t s) {
   return HP_OK;
 }
 
+// The register budget per block size: up to 256 threads a block has 128
+// registers and two or more handles' blocks share an SM; up to 448 threads 72
+// registers keep two blocks on an SM (64 x 64 x 16 slab, three handles in
+// turn: 2.4 us a step against 3.7 with 128 registers and one block); beyond,
+// one block has the SM and 96 registers.
+template <bool ANISO, bool THETA>
+static ResFn res_kernel(int threads) {
+  return threads <= RES_SMALL_THREADS ? mono_resident_kernel<ANISO, THETA, 512>
+         : threads <= RES_MID_THREADS ? mono_resident_kernel<ANISO, THETA, 896>
+                                      : mono_resident_kernel<ANISO, THETA, RES_MAX_THREADS>;
+}
+
+// Resident steps for a heart that fits on the chip at one cell per thread.
+// Where the line lies (us a step, split against resident; alone, and where
+// three handles' steps overlap on their streams): 19-point 2,258 cells
+// 6.9 / 2.6 against 3.4 / 1.2, 57,527 cells 9.5 / 4.9 against 5.8 / 3.6,
+// 90,555 cells 10.6 / 6.1 against 6.2 / 5.9; 7-point 65,539 cells 7.0 / 3.1
+// against 4.1 / 2.4, but 90,117 cells 7.5 / 3.6 against 4.5 / 4.2, so the
+// 7-point step stops at 448 threads a block.  Theta-scheme, three CG
+// iterations a step: 7,197 cells 78 / 29 against 21 / 7.4, 90,555 cells
+// 94 / 44 against 40 / 39.  At 35 iterations a step (12,473 cells) an
+// iteration takes 4.6 us against 20.
+static hp_status setup_resident(HpMono* h, const HpMonoDesc* d, cudaStream_t s) {
+  const MonoArgs& a = h->a;
+  const int64_t T = (int64_t)a.n_active_pad + a.n_pk;
+  int dev = 0, n_sm = 0, coop = 0;
+  HP_CUDA_TRY(cudaGetDevice(&dev));
+  HP_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  HP_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  const bool aniso = d->anisotropic != 0, theta = d->theta > 0.0;
+  const int most = aniso || theta ? RES_MAX_THREADS : RES_MID_THREADS;
+  if (!coop || a.n_active == 0 || T > (int64_t)n_sm * most) return HP_OK;
+  const int nq = aniso ? 18 : 6;
+  const int per = (int)((T + n_sm - 1) / n_sm);
+  h->res_threads = std::max(64, (per + 31) / 32 * 32);
+  h->res_grid = (int)((T + h->res_threads - 1) / h->res_threads);
+  if (h->res_grid > RES_MAX_BLOCKS) return HP_OK;
+  h->res_smem = (size_t)h->res_threads * (nq * 8 + (theta ? N_STATE * 4 : 0));
+  const ResFn fn = aniso ? (theta ? res_kernel<true, true>(h->res_threads)
+                                  : res_kernel<true, false>(h->res_threads))
+                         : (theta ? res_kernel<false, true>(h->res_threads)
+                                  : res_kernel<false, false>(h->res_threads));
+  HP_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)h->res_smem));
+  int fit = 0;
+  HP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, (const void*)fn, h->res_threads,
+                                                            h->res_smem));
+  if ((int64_t)fit * n_sm < h->res_grid) return HP_OK;
+  ResArgs& r = h->res_a;
+  memset(&r, 0, sizeof(r));
+  int32_t* idx = nullptr;
+  float* coef = nullptr;
+  HP_TRY_NODESTROY(al(h, &idx, (size_t)nq * a.n_active));
+  if (aniso) HP_TRY_NODESTROY(al(h, &coef, (size_t)nq * a.n_active));
+  r.idx = idx;
+  r.coef = coef;
+  // partial sums, then the arrival count, the epoch and the ticket
+  const size_t n_part = (size_t)2 * RES_MAX_BLOCKS * 8;
+  HP_TRY_NODESTROY(al(h, &r.part, n_part + 3));
+  HP_CUDA_TRY(cudaMemsetAsync(r.part, 0, (n_part + 3) * sizeof(double), s));
+  r.count = (unsigned long long*)(r.part + n_part);
+  r.epoch = r.count + 1;
+  r.ticket = (unsigned int*)(r.count + 2);
+  r.err = (int32_t*)(r.ticket + 1);
+  if (theta) {
+    r.cg_n = a.n_slots + a.n_pk;
+    HP_TRY_NODESTROY(al(h, &r.cg, (size_t)2 * r.cg_n));
+  }
+  resident_rows_kernel<<<(a.n_active + 127) / 128, 128, 0, s>>>(a, d->bi, d->bj, d->bk, nq, idx,
+                                                               coef);
+  HP_CUDA_TRY(cudaGetLastError());
+  h->res = fn;
+  return HP_OK;
+}
+
+// After a synchronising copy on s: did a barrier of a resident launch give up
+// (the state is then unusable)?
+static hp_status res_check(const HpMono* h, const char* what, cudaStream_t s) {
+  if (!h->res) return HP_OK;
+  int32_t err = 0;
+  HP_CUDA_TRY(cudaMemcpyAsync(&err, h->res_a.err, sizeof(err), cudaMemcpyDeviceToHost, s));
+  HP_CUDA_TRY(cudaStreamSynchronize(s));
+  if (err) {
+    hp::set_error("%s: a grid barrier of the resident step kernel timed out", what);
+    return HP_ERR_TIMEOUT;
+  }
+  return HP_OK;
+}
+
 extern "C" hp_status hp_mono_create(const HpMonoDesc* d, HpMono** out, void* stream) {
   HP_REQUIRE(d && out, "hp_mono_create: null argument");
   *out = nullptr;
@@ -1693,6 +1791,7 @@ extern "C" hp_status hp_mono_create(const HpMonoDesc* d, HpMono** out, void* str
   h->cn_graph = nullptr;
   h->cn_graph_steps = 0;
   h->cn_graph_stream = nullptr;
+  h->res = nullptr;
   h->anisotropic = d->anisotropic;
   h->n_steps = d->n_steps;
   h->steps_done = 0;
@@ -1836,6 +1935,13 @@ extern "C" hp_status hp_mono_create(const HpMonoDesc* d, HpMono** out, void* str
       (d->kernel == HP_MONO_KERNEL_AUTO && d->n_bricks > 0)) {
     HP_TRY(setup_split(h, se, d, s));
     if (d->theta > 0.0) HP_TRY(setup_cn(h, se, d, s));
+    if (d->kernel == HP_MONO_KERNEL_AUTO) HP_TRY(setup_resident(h, d, s));
+    if (h->cn && !h->res) {  // the tiled solve's flag copy and loop capture
+      const cudaError_t e1 = cudaMallocHost((void**)&h->cn_host, 2 * sizeof(int32_t));
+      const cudaError_t e2 = cudaStreamCreateWithFlags(&h->cn_body_stream, cudaStreamNonBlocking);
+      HP_CUDA_TRY(e1);
+      HP_CUDA_TRY(e2);
+    }
   } else if (d->kernel != HP_MONO_KERNEL_BRICK && d->n_bricks > 0) {
     HP_TRY(setup_pipe(h, se, d->anisotropic, d->kernel == HP_MONO_KERNEL_PIPELINED, s));
   }
@@ -1852,6 +1958,17 @@ extern "C" hp_status hp_mono_run(HpMono* h, int64_t n, int32_t graph_chunk, void
              "hp_mono_run: %lld steps requested, %lld remain", (long long)n,
              (long long)(h->n_steps - h->steps_done));
   cudaStream_t s = (cudaStream_t)stream;
+  if (h->res && n >= (h->cn ? 1 : RES_MIN_STEPS)) {
+    for (int64_t left = n; left > 0;) {
+      int k = (int)std::min<int64_t>(left, 1 << 16);
+      void* args[] = {&h->a, &h->cn_a, &h->res_a, &k};
+      HP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)h->res, dim3(h->res_grid),
+                                              dim3(h->res_threads), args, h->res_smem, s));
+      left -= k;
+      h->steps_done += k;
+    }
+    return HP_OK;
+  }
   if (h->cn) {
     // theta-scheme: graphs of up to 16 steps whose solve loops run on the
     // device (conditional nodes); the remainder, and the legacy default
@@ -1975,6 +2092,7 @@ extern "C" hp_status hp_mono_copy_events(HpMono* h, float* act, int32_t* n_act, 
                                   cudaMemcpyDeviceToHost, s));
       HP_CUDA_TRY(cudaStreamSynchronize(s));
     }
+    HP_TRY_NODESTROY(res_check(h, "hp_mono_copy_events", s));
     for (int64_t i = 0; i < nm; ++i) {
       const int32_t sl = h->slot_of_node[i];
       if (dn) dn[i] = c[sl];
@@ -2035,6 +2153,7 @@ extern "C" hp_status hp_mono_copy_v(HpMono* h, float* v_myo, float* v_pk, void* 
     HP_CUDA_TRY(cudaMemcpyAsync(v.data(), h->a.Vpost, v.size() * sizeof(float),
                                 cudaMemcpyDeviceToHost, s));
     HP_CUDA_TRY(cudaStreamSynchronize(s));
+    HP_TRY_NODESTROY(res_check(h, "hp_mono_copy_v", s));
     for (int64_t i = 0; i < h->a.n_myo; ++i) v_myo[i] = v[h->slot_of_node[i]];
   }
   if (v_pk && h->a.n_pk) {
@@ -2071,7 +2190,7 @@ extern "C" hp_status hp_mono_copy_state(HpMono* h, float* st_slots, float* st_pk
     HP_CUDA_TRY(cudaMemcpyAsync(st_pk, h->a.pk_state, (size_t)N_STATE * h->a.n_pk * sizeof(float),
                                 cudaMemcpyDeviceToHost, s));
   HP_CUDA_TRY(cudaStreamSynchronize(s));
-  return HP_OK;
+  return res_check(h, "hp_mono_copy_state", s);
 }
 
 extern "C" hp_status hp_mono_cn_stats(HpMono* h, int64_t* iterations, int64_t* solves,

@@ -136,7 +136,10 @@ typedef struct {
   int32_t max_events;           /* activation events kept per voxel (1..16) */
 
   /* step kernel (all give bit-identical results): HP_MONO_KERNEL_AUTO is
-   * the split step, the fastest on B200 for every compiled brick shape */
+   * the split step, the fastest on B200 for every compiled brick shape; a
+   * heart that fits on the chip at one cell per thread (about 95,000 cells)
+   * advances many steps per cooperative launch instead (same state, same
+   * results; at theta > 0 the same CG with its sums in another order) */
   int32_t kernel;
 
   /* diffusion half: theta = 0 is the explicit update above; 0 < theta <= 1
@@ -146,8 +149,7 @@ typedef struct {
    * ||r|| <= cn_tol ||rhs|| (cn_tol below 1e-7 is raised to 1e-7, FP32
    * vectors) or after cn_max_iter iterations.  pk_weight = Ai_P / Ai_M, the
    * Purkinje over the tissue membrane loading (the inner product that makes
-   * the operator symmetric).  Needs the split step (kernel AUTO or SPLIT);
-   * CUDA-graph chunks are not used (the host tests convergence). */
+   * the operator symmetric).  Needs the split step (kernel AUTO or SPLIT). */
   double theta;
   double cn_tol;
   int32_t cn_max_iter;

@@ -1703,14 +1703,10 @@ static hp_status setup_resident(HpMono* h, const HpMonoDesc* d, cudaStream_t s) 
   if (aniso) HP_TRY_NODESTROY(al(h, &coef, (size_t)nq * a.n_active));
   r.idx = idx;
   r.coef = coef;
-  // partial sums, then the arrival count, the epoch and the ticket
   const size_t n_part = (size_t)2 * RES_MAX_BLOCKS * 8;
-  HP_TRY_NODESTROY(al(h, &r.part, n_part + 3));
-  HP_CUDA_TRY(cudaMemsetAsync(r.part, 0, (n_part + 3) * sizeof(double), s));
-  r.count = (unsigned long long*)(r.part + n_part);
-  r.epoch = r.count + 1;
-  r.ticket = (unsigned int*)(r.count + 2);
-  r.err = (int32_t*)(r.ticket + 1);
+  HP_TRY_NODESTROY(al(h, &r.part, n_part + GRID_SYNC_WORDS));
+  HP_CUDA_TRY(cudaMemsetAsync(r.part, 0, (n_part + GRID_SYNC_WORDS) * sizeof(double), s));
+  r.sync = grid_sync_at(r.part + n_part);
   if (theta) {
     r.cg_n = a.n_slots + a.n_pk;
     HP_TRY_NODESTROY(al(h, &r.cg, (size_t)2 * r.cg_n));
@@ -1727,7 +1723,7 @@ static hp_status setup_resident(HpMono* h, const HpMonoDesc* d, cudaStream_t s) 
 static hp_status res_check(const HpMono* h, const char* what, cudaStream_t s) {
   if (!h->res) return HP_OK;
   int32_t err = 0;
-  HP_CUDA_TRY(cudaMemcpyAsync(&err, h->res_a.err, sizeof(err), cudaMemcpyDeviceToHost, s));
+  HP_CUDA_TRY(cudaMemcpyAsync(&err, h->res_a.sync.err, sizeof(err), cudaMemcpyDeviceToHost, s));
   HP_CUDA_TRY(cudaStreamSynchronize(s));
   if (err) {
     hp::set_error("%s: a grid barrier of the resident step kernel timed out", what);

@@ -21,24 +21,20 @@
 // round trip in turn; at 12,473 cells and 35 iterations a step the whole step
 // went from 730 to 160 us.
 #pragma once
+#include "grid_sync.cuh"
 
 namespace hp {
 
 struct ResArgs {
   const int32_t* idx;       // NQ x n_active: neighbour slot, -1 no term, -2 a term that reads 0
   const float* coef;        // NQ x n_active (19-point operator): the term's coefficient
-  unsigned long long* epoch;  // barriers passed since creation
-  unsigned int* ticket;       // blocks that are through with the launch
-  unsigned long long* count;  // arrivals since creation
+  GridSync sync;
   double* part;               // 2 x RES_MAX_BLOCKS rows of 8 partial sums
   float4* cg;               // theta: {r, q, p, D^-1} by iteration parity, 2 x cg_n
   int64_t cg_n;             // ([slots | Purkinje])
-  int32_t* err;             // set when a barrier ran out of its polls; read back with the results
 };
 constexpr int RES_MAX_BLOCKS = 160;
 constexpr int RES_BATCH = 20;  // partials in flight a thread: all of them from 64 threads on
-// A poll takes about 0.4 us, so a barrier gives up after about a second.
-constexpr int RES_MAX_POLLS = 1 << 22;
 // threads a block: register budgets (res_kernel) and the most there may be
 constexpr int RES_SMALL_THREADS = 256;
 constexpr int RES_MID_THREADS = 448;
@@ -94,16 +90,10 @@ __global__ void resident_rows_kernel(MonoArgs a, int bi, int bj, int bk, int nq,
   }
 }
 
-// Barrier over all blocks of a cooperative launch, with or without NV FP64
-// sums over all its threads; every block adds the blocks' sums in the same
-// order, so all hold the same totals.  One thread of a block arrives with a
-// release reduction on a counter and polls it with acquire loads: 0.9 us with
-// 148 blocks (a relaxed poll with a fence 1.3 us, a flag per block that every
-// block polls 7 us, clusters that arrive as one 2.2 us).  A sum costs another
-// L2 round trip for the blocks' partials, 2 us in all.  The partials
-// alternate between two sets: a block writes set e + 2 only after every block
-// has arrived at e + 1, i.e. has read e.  The counter only ever grows over the
-// handle's launches.
+// FP64 sums over all threads of the launch, in a barrier; every block adds
+// the blocks' sums in the same order, so all hold the same totals.  The
+// partials alternate between two sets: a block writes set e + 2 only after
+// every block has arrived at e + 1, i.e. has read e.  About 2 us.
 //
 // Sums run over eight values at a time: a warp halves the values a lane holds
 // at each of three exchanges (9 exchanges for 8 values instead of 40), after
@@ -131,87 +121,61 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8]) {
   return t;
 }
 
-struct GridBarrier {
-  unsigned long long epoch;
-  __device__ __forceinline__ void init(const ResArgs& r) {
-    epoch = *(volatile unsigned long long*)r.epoch;
-  }
-  // One thread: arrive, then wait for the others.  False if they did not come.
-  __device__ __forceinline__ bool arrive_wait(const ResArgs& r) {
-    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(r.count) : "memory");
-    const unsigned long long all = epoch * gridDim.x;
-    for (int k = 0; k < RES_MAX_POLLS; ++k) {
-      unsigned long long v;
-      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(r.count) : "memory");
-      if (v >= all) return true;
-    }
-    *r.err = 1;
-    return false;
-  }
-  __device__ __forceinline__ bool sync(const ResArgs& r) {
-    __shared__ int s_ok;
-    ++epoch;
-    __syncthreads();
-    if (threadIdx.x == 0) s_ok = arrive_wait(r);
-    __syncthreads();
-    return s_ok;  // rewritten only after the next barrier's first __syncthreads
-  }
-  // v (any number of values up to eight, the rest zero) becomes the totals.
-  __device__ __forceinline__ bool sum(const ResArgs& r, double (&v)[8]) {
-    __shared__ double sh[32][8];
-    __shared__ double tot[8];
-    __shared__ int s_ok;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-    const int G = gridDim.x;
-    double* part = r.part + (++epoch & 1) * (int64_t)RES_MAX_BLOCKS * 8;
-    const double t = warp_sum8(v);
-    if ((lane & 3) == 0) sh[wid][lane >> 2] = t;
-    __syncthreads();
-    if (tid < 32) {
-      // lane: value lane / 4, every fourth warp; then the four quarters
-      double s = 0.0;
-#pragma unroll
-      for (int w = 0; w < 32; w += 4)
-        if (w + (lane & 3) < nw) s += sh[w + (lane & 3)][lane >> 2];
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      if ((lane & 3) == 0) part[blockIdx.x * 8 + (lane >> 2)] = s;
-      __syncwarp();
-      if (lane == 0) s_ok = arrive_wait(r);
-    }
-    __syncthreads();
-    // the totals, in the same order in every block: thread t adds value t % 8
-    // of every (threads / 8)-th block, then the threads' sums are added
+// v (any number of values up to eight, the rest zero) becomes the totals.
+__device__ __forceinline__ bool grid_sum8(const ResArgs& r, unsigned long long& epoch,
+                                        double (&v)[8]) {
+  __shared__ double sh[32][8];
+  __shared__ double tot[8];
+  __shared__ int s_ok;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+  const int G = gridDim.x;
+  double* part = r.part + (++epoch & 1) * (int64_t)RES_MAX_BLOCKS * 8;
+  const double t = warp_sum8(v);
+  if ((lane & 3) == 0) sh[wid][lane >> 2] = t;
+  __syncthreads();
+  if (tid < 32) {
+    // lane: value lane / 4, every fourth warp; then the four quarters
     double s = 0.0;
-    const int rows = blockDim.x >> 3;
-    for (int b = tid >> 3; b < G; b += RES_BATCH * rows) {
-      double w[RES_BATCH];
 #pragma unroll
-      for (int u = 0; u < RES_BATCH; ++u)
-        w[u] = b + u * rows < G ? __ldcg(part + (b + u * rows) * 8 + (tid & 7)) : 0.0;
-#pragma unroll
-      for (int u = 0; u < RES_BATCH; ++u) s += w[u];
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 16);
-    s += __shfl_xor_sync(0xffffffffu, s, 8);
-    if (lane < 8) sh[wid][lane] = s;
-    __syncthreads();
-    if (tid < 32) {
-      double q = 0.0;
-#pragma unroll
-      for (int w = 0; w < 32; w += 4)
-        if (w + (lane & 3) < nw) q += sh[w + (lane & 3)][lane >> 2];
-      q += __shfl_xor_sync(0xffffffffu, q, 2);
-      q += __shfl_xor_sync(0xffffffffu, q, 1);
-      if ((lane & 3) == 0) tot[lane >> 2] = q;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = tot[k];
-    return s_ok;
+    for (int w = 0; w < 32; w += 4)
+      if (w + (lane & 3) < nw) s += sh[w + (lane & 3)][lane >> 2];
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    if ((lane & 3) == 0) part[blockIdx.x * 8 + (lane >> 2)] = s;
+    __syncwarp();
+    if (lane == 0) s_ok = grid_arrive_wait(r.sync, epoch);
   }
-  __device__ __forceinline__ void finish(const ResArgs& r) { *r.epoch = epoch; }
-};
+  __syncthreads();
+  // the totals, in the same order in every block: thread t adds value t % 8
+  // of every (threads / 8)-th block, then the threads' sums are added
+  double s = 0.0;
+  const int rows = blockDim.x >> 3;
+  for (int b = tid >> 3; b < G; b += RES_BATCH * rows) {
+    double w[RES_BATCH];
+#pragma unroll
+    for (int u = 0; u < RES_BATCH; ++u)
+      w[u] = b + u * rows < G ? __ldcg(part + (b + u * rows) * 8 + (tid & 7)) : 0.0;
+#pragma unroll
+    for (int u = 0; u < RES_BATCH; ++u) s += w[u];
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  if (lane < 8) sh[wid][lane] = s;
+  __syncthreads();
+  if (tid < 32) {
+    double q = 0.0;
+#pragma unroll
+    for (int w = 0; w < 32; w += 4)
+      if (w + (lane & 3) < nw) q += sh[w + (lane & 3)][lane >> 2];
+    q += __shfl_xor_sync(0xffffffffu, q, 2);
+    q += __shfl_xor_sync(0xffffffffu, q, 1);
+    if ((lane & 3) == 0) tot[lane >> 2] = q;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = tot[k];
+  return s_ok;
+}
 
 // The terms of one operator row: a field's values at its NQ neighbours,
 // loaded unconditionally (a missing term holds the cell's own slot) so that
@@ -274,8 +238,7 @@ mono_resident_kernel(MonoArgs a, CnArgs cn, ResArgs rs, int n) {
   float* scoef = smem + NQ * ld + threadIdx.x;   // NQ x ld
   float* sstate = scoef + NQ * ld;               // theta: N_STATE x ld
   const int64_t step0 = *a.d_step;
-  GridBarrier bar;
-  bar.init(rs);
+  unsigned long long epoch = *(volatile unsigned long long*)rs.sync.epoch;
 
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool tissue = i < a.n_active;
@@ -401,7 +364,7 @@ mono_resident_kernel(MonoArgs a, CnArgs cn, ResArgs rs, int n) {
         sm[0] = (double)b * b;
         sm[1] = (double)acc * acc;
       }
-      if (!bar.sum(rs, sm)) return;
+      if (!grid_sum8(rs, epoch, sm)) return;
       const double bb = sm[0];
       float alpha = 0.0f, beta = 0.0f;
       bool done = sm[1] <= cn.tol2 * bb || bb == 0.0;
@@ -444,7 +407,7 @@ mono_resident_kernel(MonoArgs a, CnArgs cn, ResArgs rs, int n) {
           sm[5] = wd * sm[2];
           sm[6] = wd * sm[3];
         }
-        if (!bar.sum(rs, sm)) return;
+        if (!grid_sum8(rs, epoch, sm)) return;
         const double pq = sm[0], rz = sm[4];
         if (!(pq > 0.0) || !isfinite(pq)) {  // breakdown: keep the current x
           ++breaks;
@@ -492,7 +455,7 @@ mono_resident_kernel(MonoArgs a, CnArgs cn, ResArgs rs, int n) {
       if (tissue) Wout[slot] = W;
       else Wpk_out[p] = W;
     }
-    if (it + 1 < n && !bar.sync(rs)) return;
+    if (it + 1 < n && !grid_sync(rs.sync, epoch)) return;
   }
   if (tissue) {
 #pragma unroll
@@ -509,12 +472,7 @@ mono_resident_kernel(MonoArgs a, CnArgs cn, ResArgs rs, int n) {
       cn.iscal[CI_BREAK] += breaks;
     }
     // the last block out advances the step and barrier counts (all have read them by then)
-    __threadfence();
-    if (atomicAdd(rs.ticket, 1u) == gridDim.x - 1) {
-      *rs.ticket = 0u;
-      bar.finish(rs);
-      *(int64_t*)a.d_step = step0 + n;
-    }
+    if (grid_last_out(rs.sync, epoch)) *(int64_t*)a.d_step = step0 + n;
   }
 }
 

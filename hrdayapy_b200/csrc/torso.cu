@@ -21,9 +21,9 @@
 // recursive FP32 residual claims convergence but the true residual does not,
 // r is replaced by the true residual and CG restarts (residual replacement).
 //
-// Reductions are deterministic: each block writes its partial, the last block
-// to arrive (atomic ticket after __threadfence) sums the partials in block
-// order and updates the scalars.  No kernel ever waits on another block.
+// The Jacobi-PCG iterations run in one cooperative launch per solve
+// (pcg_resident.cuh); the flexible-CG passes walk tissue lines, one launch
+// each.  Reductions are deterministic (partials added in block order).
 #include "hp_common.cuh"
 
 #include <math.h>
@@ -35,21 +35,10 @@
 namespace hp {
 
 constexpr int TB = 256;            // threads per block
-// resident blocks per SM the register budgets of the iteration kernels are
-// sized for (1: the compiler's choice)
-#ifndef HP_AP_MINB
-#define HP_AP_MINB 4  // pcg_ap: 64 registers (86.2 us per iteration on the full torso, 89.4 at 80)
-#endif
-#ifndef HP_K2_MINB
-#define HP_K2_MINB 1
-#endif
-#ifndef HP_PU_MINB
-#define HP_PU_MINB 1
-#endif
 constexpr int NPART = 4;           // partial sums per block
 
 enum Scal : int {
-  SC_RZ = 0, SC_PAP, SC_ALPHA, SC_BETA, SC_ALPHA_PREV, SC_ZZ, SC_ZMAX, SC_RR, SC_BB,
+  SC_RZ = 0, SC_PAP, SC_ALPHA, SC_BETA, SC_ZZ, SC_ZMAX, SC_RR, SC_BB,
   SC_TRUE_RR, SC_SRC_MEAN, SC_STAT, SC_TOL, SC_HIST0, N_SCAL = SC_HIST0 + 8
 };
 enum IScal : int {
@@ -79,10 +68,6 @@ struct TorsoArgs {
   int32_t n_lines;
   const int64_t* line_g0;
   const int32_t* line_len;
-  // the 32-cell, 128-byte aligned chunks of the padded grid that hold a
-  // tissue-line cell (each once; vectors are allocated to a multiple of 32)
-  int32_t n_chunks;
-  const int32_t* chunk;
   // label | LAB_UNIFORM when all six neighbours carry the cell's own label
   // (and, with a smoothed boundary, psi is 1 at the cell and all six),
   // | LAB_PIN at the pinned voxel
@@ -105,10 +90,6 @@ static_assert(HP_MAX_MATERIALS <= LAB_MASK + 1, "material labels must fit under 
 
 // Smoothed-boundary factor of a face: the harmonic mean of the two cells'
 // domain function, 0 when both are 0 (build_torso_grid.py:350-375).
-__device__ __forceinline__ float psi_face(float pa, float pb) {
-  const float s = pa + pb;
-  return s < 1e-30f ? 0.0f : __fdiv_rn(2.0f * pa * pb, s);
-}
 __host__ __device__ inline double psi_face64(double pa, double pb) {
   const double s = pa + pb;
   return s < 1e-30 ? 0.0 : (2.0 * pa * pb) / s;
@@ -192,7 +173,7 @@ __device__ __forceinline__ bool is_row(const TorsoArgs& a, int64_t g) {
   return a.label[g] != 0 && g != a.pin;
 }
 
-// The PCG vector kernels walk tissue lines, one warp per line (lanes over
+// The flexible-CG vector kernels walk tissue lines, one warp per line (lanes over
 // consecutive k, coalesced rows), loading a batch of LB chunks of 32 cells
 // before any arithmetic so every thread has several independent loads in
 // flight.  Air lines are never touched; inside a line the vectors are zero
@@ -216,75 +197,12 @@ __device__ __forceinline__ void for_line_batches(const TorsoArgs& a, Load&& load
   }
 }
 
-// The same over the chunk list: a warp takes U whole 32-cell chunks at a
-// time, all loads issued before any arithmetic, every access a full
-// 128-byte row segment.  Cells of a chunk outside every tissue line (air,
-// the ends of the neighbouring rows) carry zeros in every vector and invd,
-// so the updates leave them zero and they add nothing to the sums.
-template <int U, class Load, class Apply>
-__device__ __forceinline__ void for_chunk_batches(const TorsoArgs& a, Load&& load, Apply&& apply) {
-  const int lane = threadIdx.x & 31;
-  const int n_warps = gridDim.x * (TB / 32);
-  const int w = blockIdx.x * (TB / 32) + (threadIdx.x >> 5);
-  for (int c0 = w * U; c0 < a.n_chunks; c0 += n_warps * U) {
-    int64_t g[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      g[u] = c0 + u < a.n_chunks ? (int64_t)a.chunk[c0 + u] * 32 + lane : -1;
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (g[u] >= 0) load(u, g[u]);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (g[u] >= 0) apply(u, g[u]);
-  }
-}
-
-// Iteration part 1a: pending x update and p <- M^-1 r + beta p, in place
-// (every thread reads and writes only its own cells), over the chunk list
-// (measured on the full torso: 28.7 us against 31.5 us over the tissue
-// lines; the r update, with its FP64 sums, keeps the line batches of 8,
-// which measured 24.2 us against 31.3 us over chunks).
-__global__ void __launch_bounds__(TB, HP_PU_MINB) pcg_p_update(TorsoArgs a) {
-  if (a.iscal[IS_DONE]) return;
-  const double alpha_prev = a.scal[SC_ALPHA_PREV];
-  const float betaf = (float)a.scal[SC_BETA];
-  const float* __restrict__ invd = a.invd;
-  const float* __restrict__ r = a.r;
-  float* __restrict__ p = a.p0;
-  double* __restrict__ x = a.x;
-  constexpr int LB = 4;
-  float pv[LB], zv[LB];
-  if (alpha_prev != 0.0) {
-    double xv[LB];
-    for_chunk_batches<LB>(
-        a, [&](int u, int64_t g) { pv[u] = p[g]; zv[u] = invd[g] * r[g]; xv[u] = x[g]; },
-        [&](int u, int64_t g) {
-          x[g] = xv[u] + alpha_prev * (double)pv[u];
-          p[g] = zv[u] + betaf * pv[u];
-        });
-  } else {
-    for_chunk_batches<LB>(
-        a, [&](int u, int64_t g) { pv[u] = p[g]; zv[u] = invd[g] * r[g]; },
-        [&](int u, int64_t g) { p[g] = zv[u] + betaf * pv[u]; });
-  }
-}
-
-// Iteration part 1b: Ap = A p as a sum of face fluxes t (p_g - p_n) (exact
-// for equal neighbours, so a smooth p keeps its small A p instead of a
-// difference of two large sums), partial p.Ap; the last block forms alpha
-// and clears the pending x update (part 1a applied it).  One warp per
-// tissue line; all thirteen loads of a cell are issued before the sums
-// (32-bit neighbour offsets keep the addressing to one base per array).
-// The conductance table sits in shared memory (its reads diverge across a
-// warp at material boundaries).  Measured and dropped on B200 (full torso,
-// 5.8 M rows): a shared-memory 2.5-D blocked variant (8 x 32 columns
-// marching 16 planes in i, 53-56 us against 37 us here: latency-bound at one
-// plane in flight per block), two cells per thread (76 registers, 52 us) and
-// a summed-difference path for uniform cells (40 us).
-// Line SpMV core shared by the PCG and flexible-CG passes: Ap = A p over the
-// tissue lines (Ap = 0 on air and at the pin), calling cell(g, p_g, Ap_g)
-// for every cell; T is the conductance table in shared memory.
+// The flexible CG's A p, as a sum of face fluxes t (p_g - p_n) (exact for
+// equal neighbours, so a smooth p keeps its small A p instead of a difference
+// of two large sums), one warp per tissue line.  The conductance table sits
+// in shared memory (its reads diverge across a warp at material boundaries).
+// Ap = 0 on air and at the pin; cell(g, p_g, Ap_g) is called for every cell; T
+// is the conductance table in shared memory.
 //
 // Each lane takes two neighbouring cells of its line: the run is widened to
 // start on an even cell (one air cell before the first tissue cell, and at
@@ -295,12 +213,11 @@ __global__ void __launch_bounds__(TB, HP_PU_MINB) pcg_p_update(TorsoArgs a) {
 // labels are read only where a cell's six neighbours do not all share its
 // label.  Per-cell arithmetic is the same sum of face fluxes in the same
 // face order as before.
-template <bool PSI, class Cell>
+template <class Cell>
 __device__ __forceinline__ void spmv_lines(const TorsoArgs& a, const float* T, Cell&& cell) {
   const uint8_t* __restrict__ lab = a.label_u;
   const float* __restrict__ p = a.p0;
   float* __restrict__ Ap = a.Ap;
-  const float* __restrict__ psi = a.psi;
   const int sj = a.pk, si = a.pj * a.pk;   // even; the padded plane fits in 32 bits
   const int lane = threadIdx.x & 31;
   const int n_warps = gridDim.x * (TB / 32);
@@ -349,12 +266,6 @@ __device__ __forceinline__ void spmv_lines(const TorsoArgs& a, const float* T, C
           const int off[6] = {si, -si, sj, -sj, 1, -1};
 #pragma unroll
           for (int f = 0; f < 6; ++f) tf[f] = T[l * HP_MAX_MATERIALS + (le[off[f]] & M)];
-          if constexpr (PSI) {
-            const float* __restrict__ pe = psi + c + e;
-            const float pself = pe[0];
-#pragma unroll
-            for (int f = 0; f < 6; ++f) tf[f] *= psi_face(pself, pe[off[f]]);
-          }
         }
         float ap = 0.0f;
 #pragma unroll
@@ -371,12 +282,11 @@ __device__ __forceinline__ void spmv_lines(const TorsoArgs& a, const float* T, C
 
 // The same with one cell per lane, for a padded row of odd length (the
 // pair accesses need even strides).
-template <bool PSI, class Cell>
+template <class Cell>
 __device__ __forceinline__ void spmv_lines_single(const TorsoArgs& a, const float* T, Cell&& cell) {
   const uint8_t* __restrict__ lab = a.label_u;
   const float* __restrict__ p = a.p0;
   float* __restrict__ Ap = a.Ap;
-  const float* __restrict__ psi = a.psi;
   const int sj = a.pk, si = a.pj * a.pk;   // the padded plane fits in 32 bits
   const int lane = threadIdx.x & 31;
   const int n_warps = gridDim.x * (TB / 32);
@@ -404,11 +314,6 @@ __device__ __forceinline__ void spmv_lines_single(const TorsoArgs& a, const floa
       } else {
 #pragma unroll
         for (int f = 0; f < 6; ++f) tf[f] = T[l * HP_MAX_MATERIALS + (lc[off[f]] & LAB_MASK)];
-        if constexpr (PSI) {
-          const float pself = psi[g];
-#pragma unroll
-          for (int f = 0; f < 6; ++f) tf[f] *= psi_face(pself, psi[g + off[f]]);
-        }
       }
       float ap = 0.0f;
 #pragma unroll
@@ -420,133 +325,23 @@ __device__ __forceinline__ void spmv_lines_single(const TorsoArgs& a, const floa
   }
 }
 
-template <bool PAIRS, bool PSI>
-__global__ void __launch_bounds__(TB, HP_AP_MINB) pcg_ap(TorsoArgs a) {
-  __shared__ float T[HP_MAX_MATERIALS * HP_MAX_MATERIALS];
-  if (a.iscal[IS_DONE]) return;
-  for (int q = threadIdx.x; q < HP_MAX_MATERIALS * HP_MAX_MATERIALS; q += TB) T[q] = a.T32[q];
-  __syncthreads();
-  double acc[1] = {0.0};
-  auto cell = [&](int64_t, float pg, float ap) { acc[0] += (double)pg * (double)ap; };
-  if constexpr (PAIRS) spmv_lines<PSI>(a, T, cell);
-  else spmv_lines_single<PSI>(a, T, cell);
-  double tot[1];
-  if (block_reduce_last<1>(acc, 0u, a.part, a.ticket, tot) && threadIdx.x == 0) {
-    const double pAp = tot[0];
-    a.scal[SC_PAP] = pAp;
-    a.scal[SC_ALPHA_PREV] = 0.0;   // every block of part 1a applied the pending x update
-    if (!(fabs(pAp) >= 1e-30) || !isfinite(pAp)) {   // breakdown, as the reference's |pAp| < 1e-30
-      a.iscal[IS_BREAKDOWN] = isfinite(pAp) ? 1 : 0;
-      a.iscal[IS_NONFINITE] = isfinite(pAp) ? 0 : 1;
-      a.iscal[IS_DONE] = 1;
-      a.scal[SC_ALPHA] = 0.0;
-    } else {
-      a.scal[SC_ALPHA] = a.scal[SC_RZ] / pAp;
-    }
-  }
-}
+}  // namespace hp
+#include "pcg_resident.cuh"
+namespace hp {
 
-// Iteration part 2: r -= alpha Ap, z = M^-1 r, partial r.z, z.z, r.r, max|z|;
-// the last block forms beta and tests the stopping rule.
-// P99 (the reference's 'p99' metric, compute_bspm.py:195-219): stop when the
-// 0.99 quantile of |z| over the rows, linearly interpolated between order
-// statistics as torch.quantile does, is below tol.  With N rows, position
-// pos = 0.99 (N - 1), lo = floor(pos), and c rows at or above tol (their
-// order statistics start at N - c), the quantile is below tol when lo + 1 <
-// N - c, not below when lo >= N - c, and otherwise (lo = N - c - 1) equals
-// m_lt + (pos - lo) (m_ge - m_lt) with m_lt the largest |z| below tol and
-// m_ge the smallest at or above it: three reductions decide it exactly.
-// The reported statistic is that value in the last case and otherwise
-// m_lt (an upper bound of the quantile, below tol) or m_ge (a lower bound,
-// not below tol).
-template <bool P99>
-__global__ void __launch_bounds__(TB, HP_K2_MINB) pcg_k2(TorsoArgs a) {
-  if (a.iscal[IS_DONE]) return;
-  const double alpha = a.scal[SC_ALPHA];
-  const float alphaf = (float)alpha;
-  const float tolf = (float)a.scal[SC_TOL];
-  const float* __restrict__ invd = a.invd;
-  const float* __restrict__ Ap = a.Ap;
-  float* __restrict__ rv = a.r;
-  // sums r.z, z.z, r.r and max |z|; P99: r.z, count |z| >= tol, max of |z|
-  // below tol, max of -|z| at or above tol
-  double acc[4] = {0.0, 0.0, P99 ? 0.0 : 0.0, P99 ? -INFINITY : 0.0};
-  constexpr int LB = 8;
-  float rb[LB], ib[LB];
-  for_line_batches<LB>(
-      a, [&](int u, int64_t g) { rb[u] = rv[g] - alphaf * Ap[g]; ib[u] = invd[g]; },
-      [&](int u, int64_t g) {
-        const float r = rb[u];
-        rv[g] = r;
-        const float z = ib[u] * r;
-        acc[0] += (double)r * z;
-        if constexpr (P99) {
-          const float az = fabsf(z);
-          if (az >= tolf) {
-            acc[1] += 1.0;
-            acc[3] = fmax(acc[3], -(double)az);
-          } else {
-            acc[2] = fmax(acc[2], (double)az);
-          }
-        } else {
-          acc[1] += (double)z * z;
-          acc[2] += (double)r * r;
-          acc[3] = fmax(acc[3], (double)fabsf(z));
-        }
-      });
-  double tot[4];
-  if (block_reduce_last<4>(acc, P99 ? 12u : 8u, a.part, a.ticket, tot) && threadIdx.x == 0) {
-    const double rz_new = tot[0];
-    a.scal[SC_BETA] = rz_new / a.scal[SC_RZ];
-    a.scal[SC_RZ] = rz_new;
-    a.scal[SC_ALPHA_PREV] = alpha;
-    const int it = ++a.iscal[IS_ITER];
-    const int rule = a.iscal[IS_RULE];
-    double stat;
-    bool below;
-    if constexpr (P99) {
-      const double N = (double)a.n_rows, c = tot[1], m_lt = tot[2], m_ge = -tot[3];
-      const double pos = 0.99 * (N - 1.0), lo = floor(pos);
-      const double first_ge = N - c;
-      if (lo + 1.0 < first_ge) {
-        stat = m_lt;
-        below = true;
-      } else if (lo >= first_ge) {
-        stat = m_ge;
-        below = false;
-      } else {
-        stat = m_lt + (pos - lo) * (m_ge - m_lt);
-        below = stat < a.scal[SC_TOL];
-      }
-    } else {
-      a.scal[SC_ZZ] = tot[1];
-      a.scal[SC_RR] = tot[2];
-      a.scal[SC_ZMAX] = tot[3];
-      if (rule == HP_STOP_RMS) stat = sqrt(tot[1] / (double)a.n_rows);
-      else if (rule == HP_STOP_LINF) stat = tot[3];
-      else stat = sqrt(tot[2] / fmax(a.scal[SC_BB], 1e-300));  // recursive estimate
-      // REL: stop the recursion a little below tol; the true residual decides
-      const double lim = rule == HP_STOP_REL ? 0.5 * a.scal[SC_TOL] : a.scal[SC_TOL];
-      below = stat < lim;
-    }
-    a.scal[SC_STAT] = stat;
-    if (!isfinite(rz_new)) { a.iscal[IS_NONFINITE] = 1; a.iscal[IS_DONE] = 1; }
-    else if (below || it >= a.iscal[IS_MAXIT]) a.iscal[IS_DONE] = 1;
-  }
-}
-
-// x += alpha_prev * p (the pending update of the last iteration).
-__global__ void __launch_bounds__(TB) pcg_finish_x(TorsoArgs a) {
-  const double alpha = a.scal[SC_ALPHA_PREV];
-  const float* __restrict__ p = a.p0;
-  for (int64_t g = blockIdx.x * (int64_t)TB + threadIdx.x; g < a.ng;
-       g += (int64_t)gridDim.x * TB)
-    if (is_row(a, g)) a.x[g] += alpha * (double)p[g];
-}
+// What a residual pass starts: the iteration budget, stopping rule and
+// tolerance of the recursion that follows.
+struct SolveInit {
+  int32_t rule, max_iter, stag_on, iter;
+  double tol;
+};
 
 // FP64 true residual r = b - A x (written to r in FP32), and ||r||^2,
-// ||b||^2, r.M^-1 r.  Resets the CG recursion (beta = 0, no pending x).
-__global__ void __launch_bounds__(TB) true_residual(TorsoArgs a, int reset) {
+// ||b||^2, r.M^-1 r.  reset = 1 starts a CG recursion (beta = 0, the flags and
+// limits of `init`), done at once where b = 0 or the relative rule already
+// holds; 2 checks a finished one, leaving its flags (r is replaced under the
+// relative rule only); 0 evaluates the norms alone.
+__global__ void __launch_bounds__(TB) true_residual(TorsoArgs a, int reset, SolveInit init) {
   const int64_t SJ = a.pk, SI = (int64_t)a.pj * a.pk;
   double acc[3] = {0.0, 0.0, 0.0};
   for (int64_t g = blockIdx.x * (int64_t)TB + threadIdx.x; g < a.ng;
@@ -565,7 +360,7 @@ __global__ void __launch_bounds__(TB) true_residual(TorsoArgs a, int reset) {
     const double bb = (double)a.b[g];
     const double rr = bb - ax;
     const float rf = (float)rr;
-    if (reset) a.r[g] = rf;
+    if (reset == 1 || (reset == 2 && init.rule == HP_STOP_REL)) a.r[g] = rf;
     acc[0] += rr * rr;
     acc[1] += bb * bb;
     acc[2] += (double)rf * ((double)a.invd[g] * rf);
@@ -574,11 +369,18 @@ __global__ void __launch_bounds__(TB) true_residual(TorsoArgs a, int reset) {
   if (block_reduce_last<3>(acc, 0u, a.part, a.ticket, tot) && threadIdx.x == 0) {
     a.scal[SC_TRUE_RR] = tot[0];
     a.scal[SC_BB] = tot[1];
-    if (reset) {
+    if (reset == 1) {
       a.scal[SC_RZ] = tot[2];
       a.scal[SC_BETA] = 0.0;
-      a.scal[SC_ALPHA_PREV] = 0.0;
-      a.iscal[IS_DONE] = 0;
+      a.scal[SC_TOL] = init.tol;
+      const bool zero = tot[1] == 0.0;
+      const double rel = zero ? 0.0 : sqrt(tot[0] / tot[1]);
+      a.iscal[IS_DONE] = init.rule == HP_STOP_REL && (zero || rel <= init.tol) ? 1 : 0;
+      a.iscal[IS_ITER] = init.iter;
+      a.iscal[IS_RULE] = init.rule;
+      a.iscal[IS_MAXIT] = init.max_iter;
+      a.iscal[IS_BREAKDOWN] = a.iscal[IS_NONFINITE] = a.iscal[IS_STAGNANT] = a.iscal[IS_NH] = 0;
+      a.iscal[IS_STAG_ON] = init.stag_on;
     }
   }
 }
@@ -667,8 +469,7 @@ __global__ void __launch_bounds__(TB) fcg_p(TorsoArgs a, int first);
 using namespace hp;
 
 // kernels that stride over the tissue lines, in the order of HpTorso::nblk_k
-enum LineKernel : int { K_P_UPDATE = 0, K_AP, K_K2, K_FCG_SPMV, K_FCG_UPDATE, K_FCG_BETA, K_FCG_P,
-                        N_LINE_KERNELS };
+enum LineKernel : int { K_FCG_SPMV = 0, K_FCG_UPDATE, K_FCG_BETA, K_FCG_P, N_LINE_KERNELS };
 
 struct HpTorso {
   TorsoArgs a;
@@ -676,7 +477,6 @@ struct HpTorso {
   int nblk;
   int nblk_k[N_LINE_KERNELS];  // line kernels: each one's resident grid
   bool pairs;                  // stencil on cell pairs (even padded row)
-  void (*ap_fn)(TorsoArgs);
   void (*fspmv_fn)(TorsoArgs);
   int ni, nj, nk;
   int64_t n_rows;
@@ -693,17 +493,17 @@ struct HpTorso {
   float* out_dev;
   double* h_scal;   // pinned host mirrors
   int32_t* h_iscal;
-  int parity;
   bool have_x;
-  cudaGraphExec_t graph[2];
+  PcgArgs pcg;
+  int pcg_grid;
+  size_t pcg_smem;
+  void (*pcg_fn[2])(TorsoArgs, PcgArgs);   // [1]: the p99 rule
   cudaGraphExec_t fcg_graph[4];   // FCG chunk without the network / net every 1, 2, 4
   // serial number of the preconditioner handle the FCG graphs hold (not its
   // address: a destroyed handle's address can come back for a new one, whose
   // buffers the old graphs do not point to)
   uint64_t fcg_graph_pc;
   cudaStream_t fcg_graph_stream;
-  int graph_chunk;
-  cudaStream_t graph_stream;
 };
 
 template <typename T>
@@ -719,6 +519,12 @@ static hp_status tal(HpTorso* h, T** dst, size_t n) {
   return st;
 }
 
+#define HP_TRY_T(x)              \
+  do {                           \
+    hp_status _s = (x);          \
+    if (_s != HP_OK) return _s;  \
+  } while (0)
+
 #define TT_TRY(x)                \
   do {                           \
     hp_status _s = (x);          \
@@ -727,6 +533,129 @@ static hp_status tal(HpTorso* h, T** dst, size_t n) {
       return _s;                 \
     }                            \
   } while (0)
+
+template <int MODE>
+static void pcg_kernels(HpTorso* h) {
+  h->pcg_fn[0] = h->pairs ? pcg_resident<MODE, true, false> : pcg_resident<MODE, false, false>;
+  h->pcg_fn[1] = h->pairs ? pcg_resident<MODE, true, true> : pcg_resident<MODE, false, true>;
+}
+
+// The resident PCG's tables (pcg_resident.cuh) from the tissue lines, and
+// where a block keeps its vectors: all in shared memory where 36 bytes a pair
+// fit (up to about 1.7 M cells), else r alone (8 bytes, up to about 7.5 M),
+// else none.
+static hp_status setup_pcg(HpTorso* h, const std::vector<int64_t>& line_g0,
+                           const std::vector<int32_t>& line_len, const std::vector<uint8_t>& lab_u,
+                           const std::vector<float>& psi, const std::vector<float>& invd,
+                           const float* T32, int nsm, cudaStream_t s) {
+  const TorsoArgs& a = h->a;
+  PcgArgs& c = h->pcg;
+  memset(&c, 0, sizeof(c));
+  const int64_t PK = a.pk, PJ = a.pj, PK2 = (PK + 1) / 2;  // pairs a row of p
+  const int64_t SJ = PK, SI = PJ * PK;
+  const int64_t nbr[6] = {SI, -SI, SJ, -SJ, 1, -1};
+  HP_REQUIRE(a.ng / PK * PK2 < ((int64_t)1 << 31), "hp_torso_create: the grid is too large");
+  const int n_lines = (int)line_g0.size();
+  h->pcg_grid = std::max(1, std::min(nsm, PCG_MAX_BLOCKS));
+  std::vector<PcgLine> lines(n_lines);
+  std::vector<uint32_t> meta;
+  std::vector<int64_t> mixed_g;  // first cell of the mixed pairs
+  std::vector<int32_t> used(h->pcg_grid, 0);
+  meta.reserve(h->n_rows / 2 + 2 * (int64_t)n_lines);
+  auto cell = [&](int64_t g, int64_t k0, int64_t k1, int64_t k) -> int {
+    return k >= k0 && k < k1 ? lab_u[g] : 0;  // 0: not a cell of the line
+  };
+  for (int l = 0; l < n_lines; ++l) {
+    const int64_t row = line_g0[l] / PK, k0 = line_g0[l] % PK, k1 = k0 + line_len[l];
+    PcgLine& L = lines[l];
+    int32_t& at = used[(l / PCG_WARPS) % h->pcg_grid];  // lines go round by warps
+    L.p2 = (uint32_t)(row * PK2 + k0 / 2);
+    L.n2 = (int32_t)((k1 + 1) / 2 - k0 / 2);
+    L.c2 = (int32_t)meta.size();
+    L.s2 = at;
+    L.first = (int32_t)(k0 & 1);
+    L.len = line_len[l];
+    at += L.n2;
+    for (int64_t k = k0 / 2 * 2; k < k1; k += 2) {
+      const int64_t g = row * PK + k;
+      const int u0 = cell(g, k0, k1, k), u1 = cell(g + 1, k0, k1, k + 1);
+      if ((u0 & u1 & LAB_UNIFORM) && !((u0 | u1) & LAB_PIN)) {  // then both are one material
+        const int mat = u0 & LAB_MASK;
+        c.tu[mat] = T32[mat * (HP_MAX_MATERIALS + 1)];
+        c.inv[mat] = invd[g];
+        meta.push_back((uint32_t)mat);
+      } else {
+        meta.push_back(PQ_MIXED | (uint32_t)mixed_g.size());
+        mixed_g.push_back(k >= k0 ? g : g | ((int64_t)1 << 62));  // bit 62: the first cell is off the line
+        if (k + 1 >= k1) mixed_g.back() |= (int64_t)1 << 61;      // bit 61: the second is
+      }
+    }
+  }
+  c.n_lines = n_lines;
+  c.n_pairs = (int32_t)meta.size();
+  c.n_mixed = (int32_t)mixed_g.size();
+  std::vector<float> mixed((size_t)14 * mixed_g.size(), 0.0f);
+  for (size_t x = 0; x < mixed_g.size(); ++x)
+    for (int e = 0; e < 2; ++e) {
+      if ((mixed_g[x] >> (62 - e)) & 1) continue;
+      const int64_t g = (mixed_g[x] & (((int64_t)1 << 61) - 1)) + e;
+      const int l = lab_u[g] & LAB_MASK;
+      const bool row = l != 0 && !(lab_u[g] & LAB_PIN);
+      for (int f = 0; f < 6 && row; ++f) {
+        const int64_t n = g + nbr[f];
+        float t = T32[l * HP_MAX_MATERIALS + (lab_u[n] & LAB_MASK)];
+        if (!psi.empty()) {
+          const float pa = psi[g], pb = psi[n], sum = pa + pb;
+          t *= sum < 1e-30f ? 0.0f : 2.0f * pa * pb / sum;
+        }
+        mixed[((size_t)f * mixed_g.size() + x) * 2 + e] = t;
+      }
+      mixed[((size_t)6 * mixed_g.size() + x) * 2 + e] = invd[g];
+    }
+  c.sj = (uint32_t)PK2;
+  c.si = (uint32_t)(PJ * PK2);
+  const size_t np = (size_t)(a.ng / PK * PK2) * 2;
+  HP_TRY_T(tup(h, (PcgLine**)&c.line, lines.data(), lines.size(), s));
+  HP_TRY_T(tup(h, (uint32_t**)&c.meta, meta.data(), meta.size(), s));
+  if (c.n_mixed) HP_TRY_T(tup(h, (float**)&c.mixed, mixed.data(), mixed.size(), s));
+  HP_CUDA_TRY(cudaStreamSynchronize(s));  // the host vectors are temporaries
+  HP_TRY_T(tal(h, (float**)&c.p, np));
+  HP_CUDA_TRY(cudaMemsetAsync(c.p, 0, np * 4, s));
+  int dev = 0, most = 0;
+  HP_CUDA_TRY(cudaGetDevice(&dev));
+  HP_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  const size_t line_bytes =
+      (size_t)(n_lines + PCG_WARPS * h->pcg_grid - 1) / (PCG_WARPS * h->pcg_grid) * PCG_WARPS *
+      sizeof(PcgLine);
+  const size_t taken = 14 * 1024 + line_bytes;  // the reductions' static share, the lines
+  HP_REQUIRE(taken <= (size_t)most, "hp_torso_create: too many tissue lines (%d)", n_lines);
+  const size_t room = (size_t)most - taken;
+  const size_t per = ((size_t)*std::max_element(used.begin(), used.end()) + 3) / 4 * 4;
+  const int mode = per * pcg_pair_bytes(PCG_ALL) <= room ? PCG_ALL
+                   : per * pcg_pair_bytes(PCG_R) <= room ? PCG_R
+                                                         : PCG_NONE;
+  c.room = mode == PCG_NONE ? 0 : (int32_t)per;
+  h->pcg_smem = per * pcg_pair_bytes(mode) + line_bytes;
+  if (mode == PCG_ALL) pcg_kernels<PCG_ALL>(h);
+  else if (mode == PCG_R) pcg_kernels<PCG_R>(h);
+  else pcg_kernels<PCG_NONE>(h);
+  for (auto fn : h->pcg_fn)
+    HP_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)h->pcg_smem));
+  if (mode != PCG_ALL) {
+    HP_TRY_T(tal(h, &c.Ap, c.n_pairs));
+    HP_TRY_T(tal(h, &c.x, c.n_pairs));
+  }
+  if (mode == PCG_NONE) HP_TRY_T(tal(h, &c.r, c.n_pairs));
+  const size_t n_part = (size_t)2 * PCG_GROUPS * 4;
+  HP_TRY_T(tal(h, &c.part, n_part + GRID_SYNC_WORDS));
+  HP_CUDA_TRY(cudaMemsetAsync(c.part, 0, (n_part + GRID_SYNC_WORDS) * sizeof(double), s));
+  c.sync = grid_sync_at(c.part + n_part);
+  c.sync.err = a.iscal + N_ISCAL;
+  return HP_OK;
+}
+
+extern "C" hp_status hp_torso_destroy(HpTorso* h);
 
 extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* stream) {
   HP_REQUIRE(d && out, "hp_torso_create: null argument");
@@ -804,40 +733,26 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
   HpTorso* h = new HpTorso();
   memset(&h->a, 0, sizeof(h->a));
   memset(&h->s, 0, sizeof(h->s));
-  h->graph[0] = h->graph[1] = nullptr;
-  h->graph_chunk = 0;
-  h->graph_stream = nullptr;
   for (int k = 0; k < 4; ++k) h->fcg_graph[k] = nullptr;
   h->fcg_graph_pc = 0;
   h->fcg_graph_stream = nullptr;
   h->ni = ni; h->nj = nj; h->nk = nk;
   h->n_rows = n_rows;
-  h->parity = 0;
   h->have_x = false;
   TorsoArgs& a = h->a;
   TT_TRY(tup(h, (float**)&a.T32, T32, HP_MAX_MATERIALS * HP_MAX_MATERIALS, s));
   TT_TRY(tup(h, (double**)&a.T64, T64, HP_MAX_MATERIALS * HP_MAX_MATERIALS, s));
   a.ng = ng; a.pj = PJ; a.pk = PK; a.pin = pin_g; a.n_rows = n_rows;
-  // the vectors and invd extend to a multiple of 32 cells (whole chunks),
-  // zero past the grid
-  const int64_t ng32 = (ng + 31) / 32 * 32;
-  invd.resize(ng32, 0.0f);
   TT_TRY(tup(h, (uint8_t**)&a.label, lab.data(), ng, s));
-  TT_TRY(tup(h, (float**)&a.invd, invd.data(), ng32, s));
+  TT_TRY(tup(h, (float**)&a.invd, invd.data(), ng, s));
   a.psi = nullptr;
   if (d->psi) TT_TRY(tup(h, (float**)&a.psi, psi.data(), ng, s));
-  TT_TRY(tal(h, &a.r, ng32));
-  TT_TRY(tal(h, &a.p0, ng32));
-  TT_TRY(tal(h, &a.p1, ng32));
-  TT_TRY(tal(h, &a.Ap, ng32));
-  TT_TRY(tal(h, &a.x, ng32));
-  TT_TRY(tal(h, &a.b, ng32));
-  HP_CUDA_TRY(cudaMemsetAsync(a.r, 0, ng32 * 4, s));
-  HP_CUDA_TRY(cudaMemsetAsync(a.p0, 0, ng32 * 4, s));
-  HP_CUDA_TRY(cudaMemsetAsync(a.p1, 0, ng32 * 4, s));
-  HP_CUDA_TRY(cudaMemsetAsync(a.Ap, 0, ng32 * 4, s));
-  HP_CUDA_TRY(cudaMemsetAsync(a.x, 0, ng32 * 8, s));
-  HP_CUDA_TRY(cudaMemsetAsync(a.b, 0, ng32 * 4, s));
+  TT_TRY(tal(h, &a.r, ng));
+  TT_TRY(tal(h, &a.x, ng));
+  TT_TRY(tal(h, &a.b, ng));
+  HP_CUDA_TRY(cudaMemsetAsync(a.r, 0, ng * 4, s));
+  HP_CUDA_TRY(cudaMemsetAsync(a.x, 0, ng * 8, s));
+  HP_CUDA_TRY(cudaMemsetAsync(a.b, 0, ng * 4, s));
   int nsm = 148;
   {
     int dev = 0;
@@ -851,26 +766,21 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
     int o = 0;
     // cell pairs need even padded strides (an even padded row)
     h->pairs = (PK % 2) == 0;
-    // the smoothed-boundary face weights are a separate instantiation, so
-    // the sharp operator carries no psi code
-    h->ap_fn = a.psi ? (h->pairs ? pcg_ap<true, true> : pcg_ap<false, true>)
-                     : (h->pairs ? pcg_ap<true, false> : pcg_ap<false, false>);
     h->fspmv_fn = h->pairs ? fcg_spmv<true> : fcg_spmv<false>;
-    const void* fs[N_LINE_KERNELS] = {(const void*)pcg_p_update, (const void*)h->ap_fn,
-                                      (const void*)pcg_k2<false>, (const void*)h->fspmv_fn,
-                                      (const void*)fcg_update,   (const void*)fcg_beta,
-                                      (const void*)fcg_p};
+    const void* fs[N_LINE_KERNELS] = {(const void*)h->fspmv_fn, (const void*)fcg_update,
+                                      (const void*)fcg_beta, (const void*)fcg_p};
     for (int q = 0; q < N_LINE_KERNELS; ++q) {
       HP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fs[q], TB, 0));
       h->nblk_k[q] = nsm * std::min(8, std::max(o, 1));
     }
   }
-  TT_TRY(tal(h, &a.scal, N_SCAL));
-  TT_TRY(tal(h, &a.iscal, N_ISCAL));
+  // the scalars, the integer scalars and the barrier's error flag lie in one
+  // piece: one copy brings them to the host
+  TT_TRY(tal(h, &a.scal, N_SCAL + N_ISCAL / 2 + 1));
+  a.iscal = (int32_t*)(a.scal + N_SCAL);
   TT_TRY(tal(h, &a.part, (size_t)h->nblk * NPART));
   TT_TRY(tal(h, &a.ticket, 1));
-  HP_CUDA_TRY(cudaMemsetAsync(a.scal, 0, N_SCAL * 8, s));
-  HP_CUDA_TRY(cudaMemsetAsync(a.iscal, 0, N_ISCAL * 4, s));
+  HP_CUDA_TRY(cudaMemsetAsync(a.scal, 0, N_SCAL * 8 + (N_ISCAL + 1) * 4, s));
   HP_CUDA_TRY(cudaMemsetAsync(a.ticket, 0, 4, s));
   TT_TRY(tup(h, &h->grid_of_row, grid_of_row.data(), n_rows, s));
   {
@@ -892,14 +802,6 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
         }
       }
     a.n_lines = (int32_t)g0.size();
-    // chunks: the 32-cell aligned blocks that a tissue line touches, each once
-    std::vector<int32_t> chunks;
-    for (size_t L = 0; L < g0.size(); ++L) {
-      const int64_t c0 = g0[L] >> 5, c1 = (g0[L] + len[L] - 1) >> 5;
-      for (int64_t c = c0; c <= c1; ++c)
-        if (chunks.empty() || chunks.back() < (int32_t)c) chunks.push_back((int32_t)c);
-    }
-    a.n_chunks = (int32_t)chunks.size();
     std::vector<uint8_t> lab_u(lab);
     for (int64_t r = 0; r < n_rows; ++r) {
       const int64_t g = grid_of_row[r];
@@ -914,8 +816,8 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
 
     TT_TRY(tup(h, (int64_t**)&a.line_g0, g0.data(), g0.size(), s));
     TT_TRY(tup(h, (int32_t**)&a.line_len, len.data(), len.size(), s));
-    TT_TRY(tup(h, (int32_t**)&a.chunk, chunks.data(), chunks.size(), s));
-    HP_CUDA_TRY(cudaStreamSynchronize(s));  // g0 / len / chunks are stack temporaries
+    HP_CUDA_TRY(cudaStreamSynchronize(s));  // g0 / len are stack temporaries
+    TT_TRY(setup_pcg(h, g0, len, lab_u, psi, invd, T32, nsm, s));
   }
   // heart sources: segments of heart voxels per receiving row
   SrcArgs& sa = h->s;
@@ -974,8 +876,8 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
   for (int m = 0; m < d->n_read; ++m) gr[m] = grid_of_row[d->read_rows[m]];
   TT_TRY(tup(h, &h->grid_of_read, gr.data(), gr.size(), s));
   TT_TRY(tal(h, &h->out_dev, d->n_read));
-  HP_CUDA_TRY(cudaMallocHost((void**)&h->h_scal, N_SCAL * sizeof(double)));
-  HP_CUDA_TRY(cudaMallocHost((void**)&h->h_iscal, N_ISCAL * sizeof(int32_t)));
+  HP_CUDA_TRY(cudaMallocHost((void**)&h->h_scal, N_SCAL * 8 + (N_ISCAL + 1) * 4));
+  h->h_iscal = (int32_t*)(h->h_scal + N_SCAL);
   HP_CUDA_TRY(cudaStreamSynchronize(s));
   *out = h;
   return HP_OK;
@@ -983,58 +885,12 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
 
 extern "C" int64_t hp_torso_rows(const HpTorso* h) { return h ? h->n_rows : -1; }
 
-static hp_status iter_launch(HpTorso* h, int n, bool p99, cudaStream_t s) {
-  for (int q = 0; q < n; ++q) {
-    pcg_p_update<<<h->nblk_k[K_P_UPDATE], TB, 0, s>>>(h->a);
-    h->ap_fn<<<h->nblk_k[K_AP], TB, 0, s>>>(h->a);
-    if (p99) pcg_k2<true><<<h->nblk_k[K_K2], TB, 0, s>>>(h->a);
-    else pcg_k2<false><<<h->nblk_k[K_K2], TB, 0, s>>>(h->a);
-  }
-  HP_CUDA_TRY(cudaGetLastError());
-  return HP_OK;
-}
-
-// CG iterations in chunks of `chunk` (one CUDA graph per stopping-rule
-// kernel: graph[1] for the p99 rule), with the host reading the done flag
-// once per chunk.  Kernels after convergence inside a chunk return
-// immediately.
-static hp_status run_iterations(HpTorso* h, int max_iter, bool p99, cudaStream_t s) {
-  const int chunk = 8;
-  const int gi = p99 ? 1 : 0;
-  if (s == nullptr) {    // the legacy default stream cannot be captured
-    for (int done_it = 0; done_it < max_iter + chunk; done_it += chunk) {
-      hp_status st = iter_launch(h, chunk, p99, s);
-      if (st != HP_OK) return st;
-      HP_CUDA_TRY(cudaMemcpyAsync(h->h_iscal, h->a.iscal, N_ISCAL * 4, cudaMemcpyDeviceToHost, s));
-      HP_CUDA_TRY(cudaStreamSynchronize(s));
-      if (h->h_iscal[IS_DONE]) break;
-    }
-    return HP_OK;
-  }
-  if (h->graph_stream != s) {
-    for (int k = 0; k < 2; ++k) {
-      if (h->graph[k]) cudaGraphExecDestroy(h->graph[k]);
-      h->graph[k] = nullptr;
-    }
-    h->graph_stream = s;
-  }
-  if (!h->graph[gi]) {
-    cudaGraph_t g;
-    HP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    hp_status st = iter_launch(h, chunk, p99, s);
-    cudaError_t ce = cudaStreamEndCapture(s, &g);
-    if (st != HP_OK) return st;
-    HP_CUDA_TRY(ce);
-    HP_CUDA_TRY(cudaGraphInstantiate(&h->graph[gi], g, 0));
-    cudaGraphDestroy(g);
-    h->graph_chunk = chunk;
-  }
-  for (int done_it = 0; done_it < max_iter + chunk; done_it += chunk) {
-    HP_CUDA_TRY(cudaGraphLaunch(h->graph[gi], s));
-    HP_CUDA_TRY(cudaMemcpyAsync(h->h_iscal, h->a.iscal, N_ISCAL * 4, cudaMemcpyDeviceToHost, s));
-    HP_CUDA_TRY(cudaStreamSynchronize(s));
-    if (h->h_iscal[IS_DONE]) break;
-  }
+// CG iterations from the state that true_residual (or the last launch) left,
+// until the done flag: one cooperative launch.
+static hp_status run_iterations(HpTorso* h, bool p99, cudaStream_t s) {
+  void* args[] = {&h->a, &h->pcg};
+  HP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)h->pcg_fn[p99 ? 1 : 0], dim3(h->pcg_grid),
+                                          dim3(32 * PCG_WARPS), args, h->pcg_smem, s));
   return HP_OK;
 }
 
@@ -1061,69 +917,86 @@ static hp_status build_rhs(HpTorso* h, const float* vm, int vm_on_device, cudaSt
   return HP_OK;
 }
 
-static hp_status read_scalars(HpTorso* h, cudaStream_t s) {
-  HP_CUDA_TRY(cudaMemcpyAsync(h->h_scal, h->a.scal, N_SCAL * 8, cudaMemcpyDeviceToHost, s));
-  HP_CUDA_TRY(cudaMemcpyAsync(h->h_iscal, h->a.iscal, N_ISCAL * 4, cudaMemcpyDeviceToHost, s));
+// Enqueues the read-out of the current x (read-out potentials in mV).
+static hp_status readout(HpTorso* h, float* out, int out_on_device, cudaStream_t s) {
+  if (h->n_read > 0 && out) {
+    gather_out<<<(h->n_read + 255) / 256, 256, 0, s>>>(h->a.x, h->grid_of_read, h->n_read,
+                                                        out_on_device ? out : h->out_dev);
+    HP_CUDA_TRY(cudaGetLastError());
+    if (!out_on_device)
+      HP_CUDA_TRY(cudaMemcpyAsync(out, h->out_dev, h->n_read * 4, cudaMemcpyDeviceToHost, s));
+  }
+  return HP_OK;
+}
+
+// The device scalars on the host; out (may be null) receives the read-out of
+// the current x in the same wait.
+static hp_status read_scalars(HpTorso* h, cudaStream_t s, float* out = nullptr,
+                              int out_on_device = 0) {
+  HP_CUDA_TRY(cudaMemcpyAsync(h->h_scal, h->a.scal, N_SCAL * 8 + (N_ISCAL + 1) * 4,
+                              cudaMemcpyDeviceToHost, s));
+  const hp_status st = readout(h, out, out_on_device, s);
+  if (st != HP_OK) return st;
   HP_CUDA_TRY(cudaStreamSynchronize(s));
+  if (h->h_iscal[N_ISCAL]) {
+    hp::set_error("torso solve: a grid barrier timed out");
+    return HP_ERR_TIMEOUT;
+  }
   return HP_OK;
 }
 
 // Jacobi-PCG from the current x on the current b.  *result receives the
-// outcome (HP_OK, NOT_CONVERGED, STAGNATED, NONFINITE).
+// outcome (HP_OK, NOT_CONVERGED, STAGNATED, NONFINITE).  Residual, iterations
+// and the check of the result are enqueued together; the host reads the
+// scalars once per recursion and only repeats where the true residual of the
+// relative rule missed.  out (may be null) receives the read-out.
 static hp_status pcg_solve(HpTorso* h, double tol, int rule, int max_iter, HpSolveStats* stats,
-                           hp_status* result_out, cudaStream_t s) {
+                           hp_status* result_out, float* out, int out_on_device,
+                           cudaStream_t s) {
   TorsoArgs& a = h->a;
-  double tol_dev = rule == HP_STOP_REL ? tol : tol * 1e-3;   // mV -> V for the mV rules
-  HP_CUDA_TRY(cudaMemcpyAsync(a.scal + SC_TOL, &tol_dev, 8, cudaMemcpyHostToDevice, s));
-  int32_t is_init[N_ISCAL] = {0, 0, rule, max_iter, 0, 0};
-  HP_CUDA_TRY(cudaMemcpyAsync(a.iscal, is_init, sizeof(is_init), cudaMemcpyHostToDevice, s));
+  const double tol_dev = rule == HP_STOP_REL ? tol : tol * 1e-3;   // mV -> V for the mV rules
   // r = b - A x0 (warm start; x = 0 for the first frame), beta = 0
-  true_residual<<<h->nblk, TB, 0, s>>>(a, 1);
+  SolveInit init{rule, max_iter, 0, 0, tol_dev};
+  true_residual<<<h->nblk, TB, 0, s>>>(a, 1, init);
   HP_CUDA_TRY(cudaGetLastError());
   int restarts = 0;
   int total_it = 0;
   hp_status result = HP_OK;
   double rel = 0.0;
   for (;;) {
-    HP_CUDA_TRY(cudaMemcpyAsync(h->h_scal, a.scal, N_SCAL * 8, cudaMemcpyDeviceToHost, s));
-    HP_CUDA_TRY(cudaStreamSynchronize(s));
+    hp_status st = run_iterations(h, rule == HP_STOP_P99, s);
+    if (st != HP_OK) return st;
+    // the relative rule restarts from the replaced residual where it missed
+    init.max_iter = max_iter;
+    true_residual<<<h->nblk, TB, 0, s>>>(a, 2, init);
+    HP_CUDA_TRY(cudaGetLastError());
+    st = read_scalars(h, s, out, out_on_device);
+    if (st != HP_OK) return st;
     const double bb = h->h_scal[SC_BB];
     rel = bb > 0.0 ? sqrt(h->h_scal[SC_TRUE_RR] / bb) : 0.0;
-    if (bb == 0.0 && rule == HP_STOP_REL) {   // zero source: the pinned solution is 0
-      HP_CUDA_TRY(cudaMemsetAsync(a.x, 0, a.ng * 8, s));
-      rel = 0.0;
-      break;
-    }
-    if (rule == HP_STOP_REL && rel <= tol) break;
-    if (total_it >= max_iter) { result = HP_ERR_NOT_CONVERGED; break; }
-    int32_t is_run[N_ISCAL] = {0, 0, rule, max_iter - total_it, 0, 0};
-    HP_CUDA_TRY(cudaMemcpyAsync(a.iscal, is_run, sizeof(is_run), cudaMemcpyHostToDevice, s));
-    hp_status st = run_iterations(h, max_iter - total_it, rule == HP_STOP_P99, s);
-    if (st != HP_OK) return st;
-    st = read_scalars(h, s);
-    if (st != HP_OK) return st;
     const int its = h->h_iscal[IS_ITER];
     total_it += its;
-    if (its > 0) {
-      pcg_finish_x<<<h->nblk, TB, 0, s>>>(a);
-      HP_CUDA_TRY(cudaGetLastError());
+    if (bb == 0.0 && rule == HP_STOP_REL) {   // zero source: the pinned solution is 0
+      HP_CUDA_TRY(cudaMemsetAsync(a.x, 0, a.ng * 8, s));
+      st = read_scalars(h, s, out, out_on_device);
+      if (st != HP_OK) return st;
+      rel = 0.0;
+      break;
     }
     if (h->h_iscal[IS_NONFINITE]) { result = HP_ERR_NONFINITE; break; }
     if (rule != HP_STOP_REL) {
       // reference mV rules: the recursive statistic decides
-      true_residual<<<h->nblk, TB, 0, s>>>(a, 0);
-      HP_CUDA_TRY(cudaMemcpyAsync(h->h_scal, a.scal, N_SCAL * 8, cudaMemcpyDeviceToHost, s));
-      HP_CUDA_TRY(cudaStreamSynchronize(s));
-      rel = h->h_scal[SC_BB] > 0 ? sqrt(h->h_scal[SC_TRUE_RR] / h->h_scal[SC_BB]) : 0.0;
       if (!(h->h_scal[SC_STAT] < tol_dev)) result = HP_ERR_NOT_CONVERGED;
       if (h->h_iscal[IS_BREAKDOWN]) result = HP_OK;   // reference: break, return x
       break;
     }
-    // relative rule: the true residual decides; replace r and restart if needed
-    true_residual<<<h->nblk, TB, 0, s>>>(a, 1);
-    HP_CUDA_TRY(cudaGetLastError());
-    ++restarts;
+    if (its > 0 || rel > tol) ++restarts;   // a recursion ran (or broke down at once)
+    if (rel <= tol) break;
+    if (total_it >= max_iter) { result = HP_ERR_NOT_CONVERGED; break; }
     if (restarts > 50) { result = HP_ERR_STAGNATED; break; }
+    init.max_iter = max_iter - total_it;
+    true_residual<<<h->nblk, TB, 0, s>>>(a, 1, init);
+    HP_CUDA_TRY(cudaGetLastError());
   }
   if (rule == HP_STOP_REL && restarts > 0) --restarts;   // the final check is not a restart
   if (stats) {
@@ -1134,18 +1007,6 @@ static hp_status pcg_solve(HpTorso* h, double tol, int rule, int max_iter, HpSol
     stats->restarts = restarts;
   }
   *result_out = result;
-  return HP_OK;
-}
-
-static hp_status readout(HpTorso* h, float* out, int out_on_device, cudaStream_t s) {
-  if (h->n_read > 0 && out) {
-    gather_out<<<(h->n_read + 255) / 256, 256, 0, s>>>(h->a.x, h->grid_of_read, h->n_read,
-                                                        out_on_device ? out : h->out_dev);
-    if (!out_on_device)
-      HP_CUDA_TRY(cudaMemcpyAsync(out, h->out_dev, h->n_read * 4, cudaMemcpyDeviceToHost, s));
-  }
-  HP_CUDA_TRY(cudaGetLastError());
-  HP_CUDA_TRY(cudaStreamSynchronize(s));
   return HP_OK;
 }
 
@@ -1172,9 +1033,7 @@ extern "C" hp_status hp_torso_solve_frame(HpTorso* h, const float* vm, int32_t v
   hp_status st = build_rhs(h, vm, vm_on_device, s);
   if (st != HP_OK) return st;
   hp_status result = HP_OK;
-  st = pcg_solve(h, tol, rule, max_iter, stats, &result, s);
-  if (st != HP_OK) return st;
-  st = readout(h, out, out_on_device, s);
+  st = pcg_solve(h, tol, rule, max_iter, stats, &result, out, out_on_device, s);
   if (st != HP_OK) return st;
   h->have_x = true;
   return finish(result, "hp_torso_solve_frame");
@@ -1217,8 +1076,8 @@ __global__ void __launch_bounds__(TB) fcg_spmv(TorsoArgs a) {
     acc[0] += (double)pv * q;
     acc[1] += (double)pv * rv[g];
   };
-  if constexpr (PAIRS) spmv_lines<false>(a, T, cell);
-  else spmv_lines_single<false>(a, T, cell);
+  if constexpr (PAIRS) spmv_lines(a, T, cell);
+  else spmv_lines_single(a, T, cell);
   double tot[2];
   if (block_reduce_last<2>(acc, 0u, a.part, a.ticket, tot) && threadIdx.x == 0) {
     a.scal[SC_PAP] = tot[0];
@@ -1347,6 +1206,17 @@ static hp_status fcg_graph(HpTorso* h, HpPrecond* p, int use_net, cudaStream_t s
   return HP_OK;
 }
 
+// The flexible CG's own vectors, at its first solve.
+static hp_status fcg_vectors(HpTorso* h, cudaStream_t s) {
+  for (float** v : {&h->a.p0, &h->a.p1, &h->a.Ap}) {
+    if (*v) continue;
+    const hp_status st = tal(h, v, h->a.ng);
+    if (st != HP_OK) return st;
+    HP_CUDA_TRY(cudaMemsetAsync(*v, 0, h->a.ng * 4, s));
+  }
+  return HP_OK;
+}
+
 // One flexible-CG run with M (use_net selects the network term) from the
 // current x; returns with *fallback set when it did not converge within
 // fallback_iter iterations, stagnated or broke down.
@@ -1355,13 +1225,10 @@ static hp_status fcg_run(HpTorso* h, HpPrecond* p, double tol, int fallback_iter
                          cudaStream_t s) {
   TorsoArgs& a = h->a;
   *fallback = false;
-  HP_CUDA_TRY(cudaMemcpyAsync(a.scal + SC_TOL, &tol, 8, cudaMemcpyHostToDevice, s));
   // the stagnation test guards the runs with the network; the method
   // without it runs until convergence or the iteration budget
-  int32_t is_init[N_ISCAL] = {0, 0, HP_STOP_REL, fallback_iter, 0, 0};
-  is_init[IS_STAG_ON] = use_net ? 1 : 0;
-  HP_CUDA_TRY(cudaMemcpyAsync(a.iscal, is_init, sizeof(is_init), cudaMemcpyHostToDevice, s));
-  true_residual<<<h->nblk, TB, 0, s>>>(a, 1);
+  SolveInit init{HP_STOP_REL, fallback_iter, use_net ? 1 : 0, 0, tol};
+  true_residual<<<h->nblk, TB, 0, s>>>(a, 1, init);
   HP_CUDA_TRY(cudaGetLastError());
   hp_status st = read_scalars(h, s);
   if (st != HP_OK) return st;
@@ -1403,15 +1270,13 @@ static hp_status fcg_run(HpTorso* h, HpPrecond* p, double tol, int fallback_iter
     if (h->h_iscal[IS_DONE]) {
       if (h->h_scal[SC_STAT] >= 0.5 * tol) { *fallback = true; break; }   // iteration budget
       // recursive residual below tol / 2: the FP64 true residual decides
-      true_residual<<<h->nblk, TB, 0, s>>>(a, 1);
+      init.iter = it;
+      true_residual<<<h->nblk, TB, 0, s>>>(a, 1, init);
       st = read_scalars(h, s);
       if (st != HP_OK) return st;
       rel = sqrt(h->h_scal[SC_TRUE_RR] / h->h_scal[SC_BB]);
       if (rel <= tol) break;
       ++*restarts_out;
-      int32_t is_re[N_ISCAL] = {0, it, HP_STOP_REL, fallback_iter, 0, 0};
-      is_re[IS_STAG_ON] = use_net ? 1 : 0;
-      HP_CUDA_TRY(cudaMemcpyAsync(a.iscal, is_re, sizeof(is_re), cudaMemcpyHostToDevice, s));
       restart = true;
     }
   }
@@ -1448,7 +1313,8 @@ static hp_status fcg_solve(HpTorso* h, HpPrecond* p, double tol, int max_iter, i
   if (fallback) {
     HpSolveStats st2;
     hp_status r2 = HP_OK;
-    hp_status st = pcg_solve(h, tol, HP_STOP_REL, std::max(1, max_iter - it_total), &st2, &r2, s);
+    hp_status st = pcg_solve(h, tol, HP_STOP_REL, std::max(1, max_iter - it_total), &st2, &r2,
+                             nullptr, 0, s);
     if (st != HP_OK) return st;
     it_total += st2.iterations;
     rel = st2.rel_residual;
@@ -1486,29 +1352,28 @@ extern "C" hp_status hp_torso_solve_frame_fcg(HpTorso* h, HpPrecond* p, const fl
   hp_status st = build_rhs(h, vm, vm_on_device, s);
   if (st != HP_OK) return st;
   hp_status result = HP_OK;
+  st = fcg_vectors(h, s);
+  if (st != HP_OK) return st;
   st = fcg_solve(h, p, tol, max_iter, fallback_iter, use_net, stats, &result, s);
   if (st != HP_OK) return st;
   st = readout(h, out, out_on_device, s);
   if (st != HP_OK) return st;
+  HP_CUDA_TRY(cudaStreamSynchronize(s));
   h->have_x = true;
   return finish(result, "hp_torso_solve_frame_fcg");
 }
 
 namespace hp {
 // n more iterations of the current CG recursion (no restart, no stopping
-// test), then the pending x update applied so that x is the n-th iterate.
+// test): x is the n-th iterate.
 static hp_status pcg_continue(HpTorso* h, int n, cudaStream_t s) {
   TorsoArgs& a = h->a;
   const double never = 0.0;     // relative rule with tolerance 0: runs all n
   HP_CUDA_TRY(cudaMemcpyAsync(a.scal + SC_TOL, &never, 8, cudaMemcpyHostToDevice, s));
   int32_t is_run[N_ISCAL] = {0, 0, HP_STOP_REL, n, 0, 0};
   HP_CUDA_TRY(cudaMemcpyAsync(a.iscal, is_run, sizeof(is_run), cudaMemcpyHostToDevice, s));
-  hp_status st = run_iterations(h, n, false, s);
+  hp_status st = run_iterations(h, false, s);
   if (st != HP_OK) return st;
-  pcg_finish_x<<<h->nblk, TB, 0, s>>>(a);
-  HP_CUDA_TRY(cudaGetLastError());
-  const double zero = 0.0;      // the update is applied: nothing pending
-  HP_CUDA_TRY(cudaMemcpyAsync(a.scal + SC_ALPHA_PREV, &zero, 8, cudaMemcpyHostToDevice, s));
   HP_CUDA_TRY(cudaStreamSynchronize(s));   // the host scalars above are stack temporaries
   return HP_OK;
 }
@@ -1540,13 +1405,14 @@ extern "C" hp_status hp_torso_train_precond(HpTorso* h, HpPrecond* p, const floa
     if (ret != HP_OK) break;
     if (cudaMemcpyAsync(x0, a.x, a.ng * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess) { ret = HP_ERR_CUDA; break; }
     hp_status res = HP_OK;
-    ret = pcg_solve(h, tol_exact, HP_STOP_REL, 20000, nullptr, &res, s);
+    ret = pcg_solve(h, tol_exact, HP_STOP_REL, 20000, nullptr, &res, nullptr, 0, s);
     if (ret != HP_OK) break;
     if (cudaMemcpyAsync(xstar, a.x, a.ng * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess) { ret = HP_ERR_CUDA; break; }
     // one plain-PCG trajectory from the warm start; pairs at iterations ks
     // (ascending): r_k (the recursion's residual) and e_k = x* - x_k
     if (cudaMemcpyAsync(a.x, x0, a.ng * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess) { ret = HP_ERR_CUDA; break; }
-    true_residual<<<h->nblk, TB, 0, s>>>(a, 1);     // r = b - A x0, fresh recursion
+    // r = b - A x0, fresh recursion
+    true_residual<<<h->nblk, TB, 0, s>>>(a, 1, SolveInit{HP_STOP_REL, 0, 0, 0, 0.0});
     int done = 0;
     for (int kq = 0; kq < n_ks && ret == HP_OK; ++kq) {
       if (ks[kq] > done) {
@@ -1607,13 +1473,10 @@ extern "C" hp_status hp_torso_reset(HpTorso* h) {
 
 extern "C" hp_status hp_torso_destroy(HpTorso* h) {
   if (!h) return HP_OK;
-  for (int q = 0; q < 2; ++q)
-    if (h->graph[q]) cudaGraphExecDestroy(h->graph[q]);
   for (int q = 0; q < 4; ++q)
     if (h->fcg_graph[q]) cudaGraphExecDestroy(h->fcg_graph[q]);
   for (void* p : h->allocs) cudaFree(p);
   if (h->h_scal) cudaFreeHost(h->h_scal);
-  if (h->h_iscal) cudaFreeHost(h->h_iscal);
   delete h;
   return HP_OK;
 }

@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
       float* r = (float*)rs(L);
       const float* Ap = (const float*)As(L);
       const uint32_t* m = ms(L);
-#pragma unroll 4
+#pragma unroll 2
       for (int k = L.first + lane; k < L.first + L.len; k += 32) {
         const uint32_t mq = m[k >> 1];
         const float inv = (mq & PQ_MIXED)

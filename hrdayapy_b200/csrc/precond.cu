@@ -30,6 +30,7 @@
 // the error's energy that one optimal step along M(r) leaves, for the
 // residual / error pairs (r, e) the plain solver's iterates give.
 #include "hp_common.cuh"
+#include "precond_apply.cuh"
 #include "tc_conv.cuh"
 
 #include <math.h>
@@ -265,6 +266,7 @@ struct CoarseArgs {
   const float* ainv;      // nc x nc, row-major
   double* rc;
   float* zc;
+  float* zbox;            // zc by box
 };
 
 // aggregate edge lengths are powers of two: shifts instead of divisions
@@ -297,16 +299,61 @@ __global__ void __launch_bounds__(TB) coarse_restrict_kernel(CoarseArgs c, const
   if (threadIdx.x == 0) c.rc[I] = red[0];
 }
 
-// zc = A_c^-1 rc, one warp per row
-__global__ void __launch_bounds__(TB) coarse_matvec_kernel(CoarseArgs c) {
-  const int row = blockIdx.x * (TB / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
-  if (row >= c.nc) return;
-  const float* a = c.ainv + (int64_t)row * c.nc;
-  float acc = 0.0f;
-  for (int q = lane; q < c.nc; q += 32) acc += a[q] * (float)c.rc[q];
+// rc from the sums over line segments (pc::SegArgs), one warp per aggregate.
+__global__ void __launch_bounds__(TB) coarse_sum_kernel(CoarseArgs c, SegArgs g) {
+  const int I = blockIdx.x * (TB / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (I >= c.nc) return;
+  const int b = c.c_box[I];
+  const int bk = b % c.nbk, bj = (b / c.nbk) % c.nbj, bi = b / (c.nbk * c.nbj);
+  const int sh = c.ag_shift, per = c.ag / g.len;  // segments of a line in the box
+  double acc = 0.0;
+#pragma unroll 8
+  for (int t = lane; t < per << (2 * sh); t += 32) {
+    const int s = t % per, l = t / per;
+    const int i = (bi << sh) + (l >> sh), j = (bj << sh) + (l & (c.ag - 1)), k = bk * per + s;
+    if (i < c.ni && j < c.nj && k < g.n_seg)
+      acc += g.seg[((int64_t)i * g.nj + j) * g.n_seg + k];
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) c.zc[row] = acc;
+  if (lane == 0) c.rc[I] = acc;
+}
+
+// zc = A_c^-1 rc, one warp per row.  The row is read once from L2 or memory
+// (12 MB at 1,728 unknowns) in the time that allows if enough of it is in
+// flight: 32 row entries a lane are loaded before rc, staged in shared memory
+// in FP32, is even there (6.0 us against 11.7 with one load a step).
+constexpr int MV_BATCH = 32;
+__global__ void __launch_bounds__(TB) coarse_matvec_kernel(CoarseArgs c) {
+  __shared__ float rcf[HP_PC_MAX_COARSE];
+  const int row = blockIdx.x * (TB / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
+  const float* a = c.ainv + (int64_t)min(row, c.nc - 1) * c.nc;
+  float v[MV_BATCH];
+#pragma unroll
+  for (int u = 0; u < MV_BATCH; ++u) v[u] = lane + 32 * u < c.nc ? __ldg(a + lane + 32 * u) : 0.0f;
+#pragma unroll
+  for (int u = 0; u < HP_PC_MAX_COARSE / TB; ++u) {
+    const int q = threadIdx.x + u * TB;
+    if (q < c.nc) rcf[q] = (float)c.rc[q];
+  }
+  __syncthreads();
+  if (row >= c.nc) return;
+  float acc = 0.0f;
+  for (int q0 = lane; q0 < c.nc; q0 += 32 * MV_BATCH) {
+    if (q0 != lane) {
+#pragma unroll
+      for (int u = 0; u < MV_BATCH; ++u) v[u] = q0 + 32 * u < c.nc ? __ldg(a + q0 + 32 * u) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < MV_BATCH; ++u)
+      if (q0 + 32 * u < c.nc) acc = __fmaf_rn(v[u], rcf[q0 + 32 * u], acc);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) {
+    c.zc[row] = acc;
+    c.zbox[c.c_box[row]] = acc;
+  }
 }
 
 // zh[c] = coarse correction of the aggregate holding network cell c (its 8
@@ -537,6 +584,9 @@ struct HpPrecond {
   float* ainv;
   double* rc;
   float* zc;
+  float* zbox;               // zc by box
+  double* seg;               // sums of r over line segments (SegArgs)
+  int seg_len, n_seg;
 };
 
 template <typename T>
@@ -690,6 +740,12 @@ static hp_status coarse_setup(HpPrecond* h, const HpPrecondDesc* d, cudaStream_t
   HP_TRY_PC(pal(h, &h->ainv, (size_t)nc * nc));
   HP_TRY_PC(pal(h, &h->rc, nc));
   HP_TRY_PC(pal(h, &h->zc, nc));
+  HP_TRY_PC(pal(h, &h->zbox, box2c.size()));
+  HP_CUDA_TRY(cudaMemsetAsync(h->zbox, 0, box2c.size() * 4, s));
+  h->seg_len = std::min(ag, 32);
+  h->n_seg = (nk + h->seg_len - 1) / h->seg_len;
+  HP_TRY_PC(pal(h, &h->seg, (size_t)ni * nj * h->n_seg));
+  HP_CUDA_TRY(cudaMemsetAsync(h->seg, 0, (size_t)ni * nj * h->n_seg * 8, s));
   HP_CUDA_TRY(cudaMemcpyAsync(h->c_box, c_box.data(), nc * 4, cudaMemcpyHostToDevice, s));
   HP_CUDA_TRY(cudaMemcpyAsync(h->box2c, box2c.data(), box2c.size() * 4, cudaMemcpyHostToDevice, s));
   HP_CUDA_TRY(cudaMemcpyAsync(h->ainv, a32.data(), a32.size() * 4, cudaMemcpyHostToDevice, s));
@@ -853,6 +909,8 @@ extern "C" hp_status hp_precond_create(const HpPrecondDesc* d, HpPrecond** out, 
     HP_CUDA_TRY(cudaStreamSynchronize(s));
   }
   h->nc = 0;
+  h->seg = nullptr;
+  h->zbox = nullptr;
   if (d->coarse_agg >= 0) PC_TRY(coarse_setup(h, d, s));
   PC_TRY(repack(h, s));
   HP_CUDA_TRY(cudaStreamSynchronize(s));
@@ -893,7 +951,7 @@ static CoarseArgs coarse_args(const HpPrecond* h, const uint8_t* label) {
   int sh = 0;
   while ((1 << sh) < h->ag) ++sh;
   return CoarseArgs{h->ni, h->nj, h->nk, h->pj, h->pk, h->ag, sh, h->nbj, h->nbk, h->nc, h->pin,
-                    label, h->c_box, h->box2c, h->ainv, h->rc, h->zc};
+                    label, h->c_box, h->box2c, h->ainv, h->rc, h->zc, h->zbox};
 }
 
 // zc = A_c^-1 Q^T r (no-op without a coarse level)
@@ -948,14 +1006,39 @@ hp_status precond_forward(HpPrecond* h, const uint8_t* label, const float* invd,
 
 uint64_t precond_serial(const HpPrecond* h) { return h->serial; }
 
-hp_status precond_apply(HpPrecond* h, const uint8_t* label, const float* invd, const float* r,
-                        float* z, int use_net, cudaStream_t s) {
-  hp_status cst = coarse_solve(h, label, r, s);
-  if (cst != HP_OK) return cst;
-  if (use_net) {
-    hp_status st = precond_forward(h, label, invd, r, s);
-    if (st != HP_OK) return st;
+SegArgs precond_segments(const HpPrecond* h) {
+  return SegArgs{h->nc > 0 ? h->seg : nullptr, h->seg_len, h->n_seg, h->nj};
+}
+
+ZArgs precond_z(const HpPrecond* h, int use_net) {
+  const CoarseArgs c = coarse_args(h, nullptr);
+  return ZArgs{h->omega, h->nc > 0 ? h->zbox : nullptr, c.ag_shift, h->nbj, h->nbk,
+               use_net ? h->y : nullptr, h->scale, h->L[1].H, h->L[1].W};
+}
+
+hp_status precond_update(HpPrecond* h, const uint8_t* label, const float* invd, const float* r,
+                         int use_net, cudaStream_t s) {
+  if (h->nc > 0) {
+    const CoarseArgs c = coarse_args(h, label);
+    const int grid = (h->nc + TB / 32 - 1) / (TB / 32);
+    coarse_sum_kernel<<<grid, TB, 0, s>>>(c, precond_segments(h));
+    coarse_matvec_kernel<<<grid, TB, 0, s>>>(c);
+    HP_CUDA_TRY(cudaGetLastError());
   }
+  return use_net ? precond_forward(h, label, invd, r, s) : HP_OK;
+}
+
+hp_status precond_begin(HpPrecond* h, const uint8_t* label, const float* invd, const float* r,
+                        int use_net, cudaStream_t s) {
+  const hp_status st = coarse_solve(h, label, r, s);
+  if (st != HP_OK || !use_net) return st;
+  return precond_forward(h, label, invd, r, s);
+}
+
+static hp_status precond_apply(HpPrecond* h, const uint8_t* label, const float* invd,
+                               const float* r, float* z, int use_net, cudaStream_t s) {
+  const hp_status st = precond_begin(h, label, invd, r, use_net, s);
+  if (st != HP_OK) return st;
   ProlongArgs pa{coarse_args(h, label), h->pj, h->pk, h->ng, h->pin, label, invd, r, h->y,
                  h->scale, h->omega, h->L[1], use_net};
   prolong_kernel<<<dim3(h->pj, (unsigned)(h->ng / ((int64_t)h->pj * h->pk))), TB, 0, s>>>(pa, z);

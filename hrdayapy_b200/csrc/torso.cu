@@ -25,6 +25,7 @@
 // (pcg_resident.cuh); the flexible-CG passes walk tissue lines, one launch
 // each.  Reductions are deterministic (partials added in block order).
 #include "hp_common.cuh"
+#include "precond_apply.cuh"
 
 #include <math.h>
 #include <stdint.h>
@@ -36,6 +37,7 @@ namespace hp {
 
 constexpr int TB = 256;            // threads per block
 constexpr int NPART = 4;           // partial sums per block
+constexpr int FCG_SPMV_BLOCKS = 4; // blocks a multiprocessor of the flexible CG's A p (fixes its sums' order)
 
 enum Scal : int {
   SC_RZ = 0, SC_PAP, SC_ALPHA, SC_BETA, SC_ZZ, SC_ZMAX, SC_RR, SC_BB,
@@ -53,7 +55,6 @@ struct TorsoArgs {
   const float* invd;
   float* r;
   float* p0;
-  float* p1;
   float* Ap;
   double* x;
   float* b;
@@ -66,23 +67,20 @@ struct TorsoArgs {
   // tissue lines: the k-run from the first to the last tissue cell of every
   // (i, j) line that has one (air inside a run is allowed)
   int32_t n_lines;
-  const int64_t* line_g0;
-  const int32_t* line_len;
-  // label | LAB_UNIFORM when all six neighbours carry the cell's own label
-  // (and, with a smoothed boundary, psi is 1 at the cell and all six),
-  // | LAB_PIN at the pinned voxel
-  const uint8_t* label_u;
+  const int4* line;    // row of the padded grid, unpadded k of its first and past its last cell,
+                       // unpadded i
   // smoothed-boundary domain function per padded cell (0 off the rows), or
   // null for the sharp boundary
   const float* psi;
-  // this handle's conductance tables (harmonic-mean face conductance / h^2,
-  // HP_MAX_MATERIALS x HP_MAX_MATERIALS, FP32 for the iteration, FP64 for
-  // the true residual): per handle, so that handles with different
-  // conductivities can live side by side on one device
-  const float* T32;
+  // this handle's FP64 conductance table of the true residual (harmonic-mean
+  // face conductance / h^2, HP_MAX_MATERIALS x HP_MAX_MATERIALS): per handle,
+  // so that handles with different conductivities can live side by side
   const double* T64;
 };
 
+// flags over the host copy of the labels: all six neighbours carry the cell's
+// own label (and, with a smoothed boundary, psi is 1 at the cell and all six);
+// the pinned voxel
 constexpr int LAB_UNIFORM = 0x80;
 constexpr int LAB_PIN = 0x40;
 constexpr int LAB_MASK = 0x3F;  // the material label (< HP_MAX_MATERIALS)
@@ -171,158 +169,6 @@ __device__ bool block_reduce_last(double (&v)[NV], uint32_t max_mask, double* pa
 
 __device__ __forceinline__ bool is_row(const TorsoArgs& a, int64_t g) {
   return a.label[g] != 0 && g != a.pin;
-}
-
-// The flexible-CG vector kernels walk tissue lines, one warp per line (lanes over
-// consecutive k, coalesced rows), loading a batch of LB chunks of 32 cells
-// before any arithmetic so every thread has several independent loads in
-// flight.  Air lines are never touched; inside a line the vectors are zero
-// on air cells and at the pinned voxel (r, p, x start at 0 and only row
-// cells are ever written non-zero; invd is 0 there), so no labels are read.
-template <int LB, class Load, class Apply>
-__device__ __forceinline__ void for_line_batches(const TorsoArgs& a, Load&& load, Apply&& apply) {
-  const int lane = threadIdx.x & 31;
-  const int n_warps = gridDim.x * (TB / 32);
-  for (int L = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); L < a.n_lines; L += n_warps) {
-    const int64_t g0 = a.line_g0[L];
-    const int len = a.line_len[L];
-    for (int k0 = lane; k0 < len; k0 += 32 * LB) {
-#pragma unroll
-      for (int u = 0; u < LB; ++u)
-        if (k0 + 32 * u < len) load(u, g0 + k0 + 32 * u);
-#pragma unroll
-      for (int u = 0; u < LB; ++u)
-        if (k0 + 32 * u < len) apply(u, g0 + k0 + 32 * u);
-    }
-  }
-}
-
-// The flexible CG's A p, as a sum of face fluxes t (p_g - p_n) (exact for
-// equal neighbours, so a smooth p keeps its small A p instead of a difference
-// of two large sums), one warp per tissue line.  The conductance table sits
-// in shared memory (its reads diverge across a warp at material boundaries).
-// Ap = 0 on air and at the pin; cell(g, p_g, Ap_g) is called for every cell; T
-// is the conductance table in shared memory.
-//
-// Each lane takes two neighbouring cells of its line: the run is widened to
-// start on an even cell (one air cell before the first tissue cell, and at
-// most one after the last), so p, Ap and the labels of the pair move as one
-// 8-byte / 2-byte access at the cell and at its four i / j neighbours (the
-// padded plane and row strides are even), and the +-k neighbours come from
-// the adjacent lanes by shuffles (lanes 0 and 31 load theirs).  Neighbour
-// labels are read only where a cell's six neighbours do not all share its
-// label.  Per-cell arithmetic is the same sum of face fluxes in the same
-// face order as before.
-template <class Cell>
-__device__ __forceinline__ void spmv_lines(const TorsoArgs& a, const float* T, Cell&& cell) {
-  const uint8_t* __restrict__ lab = a.label_u;
-  const float* __restrict__ p = a.p0;
-  float* __restrict__ Ap = a.Ap;
-  const int sj = a.pk, si = a.pj * a.pk;   // even; the padded plane fits in 32 bits
-  const int lane = threadIdx.x & 31;
-  const int n_warps = gridDim.x * (TB / 32);
-  constexpr int M = LAB_MASK;
-  for (int L = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); L < a.n_lines; L += n_warps) {
-    const int64_t g0 = a.line_g0[L];
-    const int64_t ga = g0 & ~(int64_t)1;                  // even start
-    const int npairs = (int)((g0 + a.line_len[L] - ga + 1) >> 1);
-    for (int q0 = 0; q0 < npairs; q0 += 32) {
-      const int q = q0 + lane;
-      const bool on = q < npairs;
-      const int64_t c = ga + 2 * (int64_t)q;            // first cell of the pair
-      float2 pc = make_float2(0.0f, 0.0f), pip = pc, pim = pc, pjp = pc, pjm = pc;
-      uchar2 lc = make_uchar2(0, 0);
-      if (on) {
-        pc = *(const float2*)(p + c);
-        pip = *(const float2*)(p + c + si);
-        pim = *(const float2*)(p + c - si);
-        pjp = *(const float2*)(p + c + sj);
-        pjm = *(const float2*)(p + c - sj);
-        lc = *(const uchar2*)(lab + c);
-      }
-      // -k of the first cell = second cell of the lane below; +k of the
-      // second cell = first cell of the lane above
-      float km = __shfl_up_sync(0xffffffffu, pc.y, 1);
-      float kp = __shfl_down_sync(0xffffffffu, pc.x, 1);
-      if (on && lane == 0) km = p[c - 1];
-      if (on && lane == 31) kp = p[c + 2];
-      if (!on) continue;
-      const float pv[2] = {pc.x, pc.y};
-      const float pn0[2][6] = {{pip.x, pim.x, pjp.x, pjm.x, pc.y, km},
-                               {pip.y, pim.y, pjp.y, pjm.y, kp, pc.x}};
-      const int lf[2] = {lc.x, lc.y};
-      float ap2[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int l = lf[e] & M;
-        // face conductances: one table entry inside a material region
-        float tf[6];
-        if (lf[e] & LAB_UNIFORM) {
-          const float t = T[l * (HP_MAX_MATERIALS + 1)];
-#pragma unroll
-          for (int f = 0; f < 6; ++f) tf[f] = t;
-        } else {
-          const uint8_t* __restrict__ le = lab + c + e;
-          const int off[6] = {si, -si, sj, -sj, 1, -1};
-#pragma unroll
-          for (int f = 0; f < 6; ++f) tf[f] = T[l * HP_MAX_MATERIALS + (le[off[f]] & M)];
-        }
-        float ap = 0.0f;
-#pragma unroll
-        for (int f = 0; f < 6; ++f) ap += tf[f] * (pv[e] - pn0[e][f]);
-        if (l == 0 || (lf[e] & LAB_PIN)) ap = 0.0f;
-        ap2[e] = ap;
-      }
-      *(float2*)(Ap + c) = make_float2(ap2[0], ap2[1]);
-      cell(c, pv[0], ap2[0]);
-      cell(c + 1, pv[1], ap2[1]);
-    }
-  }
-}
-
-// The same with one cell per lane, for a padded row of odd length (the
-// pair accesses need even strides).
-template <class Cell>
-__device__ __forceinline__ void spmv_lines_single(const TorsoArgs& a, const float* T, Cell&& cell) {
-  const uint8_t* __restrict__ lab = a.label_u;
-  const float* __restrict__ p = a.p0;
-  float* __restrict__ Ap = a.Ap;
-  const int sj = a.pk, si = a.pj * a.pk;   // the padded plane fits in 32 bits
-  const int lane = threadIdx.x & 31;
-  const int n_warps = gridDim.x * (TB / 32);
-  for (int L = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); L < a.n_lines; L += n_warps) {
-    const int64_t g0 = a.line_g0[L];
-    const int len = a.line_len[L];
-    for (int k = lane; k < len; k += 32) {
-      const int64_t g = g0 + k;
-      const uint8_t* __restrict__ lc = lab + g;
-      const float* __restrict__ pc = p + g;
-      const int off[6] = {si, -si, sj, -sj, 1, -1};
-      const int lf = lc[0];
-      const int l = lf & LAB_MASK;
-      const float pg = pc[0];
-      float pn[6];
-#pragma unroll
-      for (int f = 0; f < 6; ++f) pn[f] = pc[off[f]];
-      // inside a material region every face has the same conductance: one
-      // table entry, and the neighbours' labels are read only at boundaries
-      float tf[6];
-      if (lf & LAB_UNIFORM) {
-        const float t = T[l * (HP_MAX_MATERIALS + 1)];
-#pragma unroll
-        for (int f = 0; f < 6; ++f) tf[f] = t;
-      } else {
-#pragma unroll
-        for (int f = 0; f < 6; ++f) tf[f] = T[l * HP_MAX_MATERIALS + (lc[off[f]] & LAB_MASK)];
-      }
-      float ap = 0.0f;
-#pragma unroll
-      for (int f = 0; f < 6; ++f) ap += tf[f] * (pg - pn[f]);
-      if (l == 0 || (lf & LAB_PIN)) ap = 0.0f;
-      Ap[g] = ap;
-      cell(g, pg, ap);
-    }
-  }
 }
 
 }  // namespace hp
@@ -458,11 +304,10 @@ __global__ void gather_rows_f(const float* b, const int64_t* grid_of_row, int64_
 }
 
 // flexible-CG passes (defined with the FCG driver below)
-template <bool PAIRS>
-__global__ void __launch_bounds__(TB) fcg_spmv(TorsoArgs a);
-__global__ void __launch_bounds__(TB) fcg_update(TorsoArgs a);
-__global__ void __launch_bounds__(TB) fcg_beta(TorsoArgs a);
-__global__ void __launch_bounds__(TB) fcg_p(TorsoArgs a, int first);
+__global__ void __launch_bounds__(TB, 4) fcg_spmv(TorsoArgs a, PcgArgs c);
+__global__ void __launch_bounds__(TB) fcg_update(TorsoArgs a, pc::SegArgs seg);
+__global__ void __launch_bounds__(TB) fcg_beta(TorsoArgs a, pc::ZArgs z);
+__global__ void __launch_bounds__(TB) fcg_p(TorsoArgs a, pc::ZArgs z, int first);
 
 }  // namespace hp
 
@@ -477,7 +322,6 @@ struct HpTorso {
   int nblk;
   int nblk_k[N_LINE_KERNELS];  // line kernels: each one's resident grid
   bool pairs;                  // stencil on cell pairs (even padded row)
-  void (*fspmv_fn)(TorsoArgs);
   int ni, nj, nk;
   int64_t n_rows;
   std::vector<void*> allocs;
@@ -740,13 +584,18 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
   h->n_rows = n_rows;
   h->have_x = false;
   TorsoArgs& a = h->a;
-  TT_TRY(tup(h, (float**)&a.T32, T32, HP_MAX_MATERIALS * HP_MAX_MATERIALS, s));
   TT_TRY(tup(h, (double**)&a.T64, T64, HP_MAX_MATERIALS * HP_MAX_MATERIALS, s));
   a.ng = ng; a.pj = PJ; a.pk = PK; a.pin = pin_g; a.n_rows = n_rows;
   TT_TRY(tup(h, (uint8_t**)&a.label, lab.data(), ng, s));
   TT_TRY(tup(h, (float**)&a.invd, invd.data(), ng, s));
   a.psi = nullptr;
   if (d->psi) TT_TRY(tup(h, (float**)&a.psi, psi.data(), ng, s));
+  // the flexible CG's own vectors, where a preconditioner can be made at all
+  if (!d->psi && ni % 8 == 0 && nj % 8 == 0 && nk % 256 == 0)
+    for (float** v : {&a.p0, &a.Ap}) {
+      TT_TRY(tal(h, v, ng));
+      HP_CUDA_TRY(cudaMemsetAsync(*v, 0, ng * 4, s));
+    }
   TT_TRY(tal(h, &a.r, ng));
   TT_TRY(tal(h, &a.x, ng));
   TT_TRY(tal(h, &a.b, ng));
@@ -766,13 +615,13 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
     int o = 0;
     // cell pairs need even padded strides (an even padded row)
     h->pairs = (PK % 2) == 0;
-    h->fspmv_fn = h->pairs ? fcg_spmv<true> : fcg_spmv<false>;
-    const void* fs[N_LINE_KERNELS] = {(const void*)h->fspmv_fn, (const void*)fcg_update,
+    const void* fs[N_LINE_KERNELS] = {(const void*)fcg_spmv, (const void*)fcg_update,
                                       (const void*)fcg_beta, (const void*)fcg_p};
     for (int q = 0; q < N_LINE_KERNELS; ++q) {
       HP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fs[q], TB, 0));
       h->nblk_k[q] = nsm * std::min(8, std::max(o, 1));
     }
+    h->nblk_k[K_FCG_SPMV] = nsm * FCG_SPMV_BLOCKS;
   }
   // the scalars, the integer scalars and the barrier's error flag lie in one
   // piece: one copy brings them to the host
@@ -812,11 +661,14 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
       if (uni) lab_u[g] |= (uint8_t)LAB_UNIFORM;
     }
     lab_u[pin_g] |= (uint8_t)LAB_PIN;
-    TT_TRY(tup(h, (uint8_t**)&a.label_u, lab_u.data(), lab_u.size(), s));
 
-    TT_TRY(tup(h, (int64_t**)&a.line_g0, g0.data(), g0.size(), s));
-    TT_TRY(tup(h, (int32_t**)&a.line_len, len.data(), len.size(), s));
-    HP_CUDA_TRY(cudaStreamSynchronize(s));  // g0 / len are stack temporaries
+    std::vector<int4> line(g0.size());
+    for (size_t L = 0; L < g0.size(); ++L) {
+      const int row = (int)(g0[L] / PK), k0 = (int)(g0[L] % PK) - 1;
+      line[L] = make_int4(row, k0, k0 + len[L], row / PJ - 1);
+    }
+    TT_TRY(tup(h, (int4**)&a.line, line.data(), line.size(), s));
+    HP_CUDA_TRY(cudaStreamSynchronize(s));  // line is a stack temporary
     TT_TRY(setup_pcg(h, g0, len, lab_u, psi, invd, T32, nsm, s));
   }
   // heart sources: segments of heart voxels per receiving row
@@ -1055,29 +907,59 @@ extern "C" hp_status hp_torso_arrays(HpTorso* h, HpTorsoArrays* o) {
 // ------------------------------------------------------------ flexible CG
 
 namespace hp {
-namespace pc {
-hp_status precond_apply(HpPrecond* h, const uint8_t* label, const float* invd, const float* r,
-                        float* z, int use_net, cudaStream_t s);
-uint64_t precond_serial(const HpPrecond* h);
-}
 
-// q = A p (p in p0), partial p.q and p.r; last block: alpha = p.r / p.q.
-// The flexible-CG passes walk the tissue lines like the PCG ones (the
-// preconditioner output z is zero on air and at the pin as well).
-template <bool PAIRS>
-__global__ void __launch_bounds__(TB) fcg_spmv(TorsoArgs a) {
-  __shared__ float T[HP_MAX_MATERIALS * HP_MAX_MATERIALS];
+// q = A p (p in p0), partial p.q and p.r; last block: alpha = p.r / p.q.  On
+// the resident PCG's pair tables (41 us on the full torso where every cell
+// decoded its label, 31 here), one warp per tissue line; the order of the
+// two sums is fixed like the PCG's (see pcg_resident.cuh), so the grid is.
+// (The preconditioners need an even padded row, so pairs are aligned.)
+__global__ void __launch_bounds__(TB, 4) fcg_spmv(TorsoArgs a, PcgArgs c) {
+  __shared__ float s_t[HP_MAX_MATERIALS];
   if (a.iscal[IS_DONE]) return;
-  for (int q = threadIdx.x; q < HP_MAX_MATERIALS * HP_MAX_MATERIALS; q += TB) T[q] = a.T32[q];
+  if (threadIdx.x < HP_MAX_MATERIALS) s_t[threadIdx.x] = c.tu[threadIdx.x];
   __syncthreads();
-  const float* __restrict__ rv = a.r;
+  const int lane = threadIdx.x & 31;
+  const int n_warps = gridDim.x * (TB / 32);
+  const int64_t sj = a.pk / 2, si = (int64_t)a.pj * sj;
   double acc[2] = {0.0, 0.0};
-  auto cell = [&](int64_t g, float pv, float q) {
-    acc[0] += (double)pv * q;
-    acc[1] += (double)pv * rv[g];
-  };
-  if constexpr (PAIRS) spmv_lines(a, T, cell);
-  else spmv_lines_single(a, T, cell);
+  for (int l = blockIdx.x * (TB / 32) + (threadIdx.x >> 5); l < c.n_lines; l += n_warps) {
+    const PcgLine L = c.line[l];
+    const int64_t g2 = (int64_t)(L.p2 / c.sj) * sj + L.p2 % c.sj;  // first pair in the padded grid
+    const float2* __restrict__ p = (const float2*)a.p0 + g2;
+    const float2* __restrict__ rv = (const float2*)a.r + g2;
+    float2* __restrict__ Ap = (float2*)a.Ap + g2;
+    const uint32_t* __restrict__ m = c.meta + L.c2;
+    for (int q = lane; q < L.n2; q += 32) {
+      const uint32_t mq = m[q];
+      const float2 pc = p[q], ip = p[q + si], im = p[q - si], jp = p[q + sj], jm = p[q - sj];
+      const float km = ((const float*)p)[2 * q - 1], kp = ((const float*)p)[2 * q + 2];
+      const float2 rq = rv[q];
+      const float pv[2] = {pc.x, pc.y};
+      const float nb[6][2] = {{ip.x, ip.y}, {im.x, im.y}, {jp.x, jp.y},
+                              {jm.x, jm.y}, {pc.y, kp},   {km, pc.x}};
+      float ap[2] = {0.0f, 0.0f};
+      if (mq & PQ_MIXED) {
+        const float2* __restrict__ W = c.mixed + (mq & ~PQ_MIXED);
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+          const float2 w = W[f * (int64_t)c.n_mixed];
+          ap[0] = __fmaf_rn(w.x, __fsub_rn(pv[0], nb[f][0]), ap[0]);
+          ap[1] = __fmaf_rn(w.y, __fsub_rn(pv[1], nb[f][1]), ap[1]);
+        }
+      } else {
+        const float w = s_t[mq];
+#pragma unroll
+        for (int f = 0; f < 6; ++f)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) ap[e] = __fmaf_rn(w, __fsub_rn(pv[e], nb[f][e]), ap[e]);
+      }
+      Ap[q] = make_float2(ap[0], ap[1]);
+      acc[0] += (double)pv[0] * (double)ap[0];
+      acc[1] += (double)pv[0] * (double)rq.x;
+      acc[0] += (double)pv[1] * (double)ap[1];
+      acc[1] += (double)pv[1] * (double)rq.y;
+    }
+  }
   double tot[2];
   if (block_reduce_last<2>(acc, 0u, a.part, a.ticket, tot) && threadIdx.x == 0) {
     a.scal[SC_PAP] = tot[0];
@@ -1092,8 +974,47 @@ __global__ void __launch_bounds__(TB) fcg_spmv(TorsoArgs a) {
   }
 }
 
-// x += alpha p, r -= alpha q, partial r.r; last block: recursive stat, done test
-__global__ void __launch_bounds__(TB) fcg_update(TorsoArgs a) {
+// The flexible-CG vector passes below take pieces of 32 LB cells of a tissue
+// line that start on a multiple of 32 LB of the unpadded k, one warp per piece
+// (whole lines left the last of 5 rounds of the full torso's warps a tenth
+// full), all loads of a piece issued before any arithmetic: load(u, g) on the
+// line's cells, apply(u, g, on) by all lanes (on: a cell of the line), then
+// done(i, j, k) with the unpadded line and the piece's first k.
+template <int LB, class Load, class Apply, class Done>
+__device__ __forceinline__ void for_aligned_lines(const TorsoArgs& a, Load&& load, Apply&& apply,
+                                                  Done&& done) {
+  const int lane = threadIdx.x & 31;
+  const int n_warps = gridDim.x * (TB / 32);
+  const int per = (a.pk + 32 * LB - 3) / (32 * LB);  // pieces of a row of pk - 2 cells
+  const int n = a.n_lines * per;
+  int w = blockIdx.x * (TB / 32) + (threadIdx.x >> 5);
+  int4 next = w < n ? a.line[w / per] : make_int4(0, 0, 0, 0);  // one piece ahead
+  for (; w < n; w += n_warps) {
+    const int4 line = next;
+    if (w + n_warps < n) next = a.line[(w + n_warps) / per];
+    const int k0 = w % per * 32 * LB, first = line.y, end = line.z;
+    if (k0 >= end || k0 + 32 * LB <= first) continue;
+    const int64_t base = (int64_t)line.x * a.pk + 1;
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      const int k = k0 + 32 * u + lane;
+      if (k >= first && k < end) load(u, base + k);
+    }
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      const int k = k0 + 32 * u + lane;
+      apply(u, base + k, k >= first && k < end);
+    }
+    done(line.w, line.x - (line.w + 1) * a.pj - 1, k0);
+  }
+}
+
+// x += alpha p, r -= alpha q, partial r.r, and the sums of r over the coarse
+// level's line segments (while r is in registers: a pass over r of its own
+// took 35 us on the full torso); last block: recursive stat, done test.
+// Bound by memory: 32 bytes a cell, 43 us cold on the full torso (29 us at the
+// copy bandwidth).
+__global__ void __launch_bounds__(TB) fcg_update(TorsoArgs a, pc::SegArgs seg) {
   if (a.iscal[IS_DONE]) return;
   const double alpha = a.scal[SC_ALPHA];
   const float af = (float)alpha;
@@ -1103,19 +1024,37 @@ __global__ void __launch_bounds__(TB) fcg_update(TorsoArgs a) {
   double* __restrict__ x = a.x;
   double acc[1] = {0.0};
   constexpr int LB = 4;
+  const int lane = threadIdx.x & 31;
   float pb[LB], rb[LB];
-  double xb[LB];
-  for_line_batches<LB>(
+  double xb[LB], sb[LB];
+  for_aligned_lines<LB>(
       a,
       [&](int u, int64_t g) {
         pb[u] = p[g];
         xb[u] = x[g];
         rb[u] = rv[g] - af * Ap[g];
       },
-      [&](int u, int64_t g) {
-        x[g] = xb[u] + alpha * (double)pb[u];
-        rv[g] = rb[u];
-        acc[0] += (double)rb[u] * rb[u];
+      [&](int u, int64_t g, bool on) {
+        sb[u] = 0.0;
+        if (on) {
+          x[g] = xb[u] + alpha * (double)pb[u];
+          rv[g] = rb[u];
+          sb[u] = (double)rb[u];
+          acc[0] += sb[u] * sb[u];
+        }
+      },
+      [&](int i, int j, int k) {
+        if (!seg.seg) return;
+        // four steps' sums at once: lanes exchange two, then one of them, so
+        // that lane l goes on with step l % 4; then over the segment
+        const bool b0 = lane & 1, b1 = lane & 2;
+        double t0 = (b0 ? sb[1] : sb[0]) + __shfl_xor_sync(0xffffffffu, b0 ? sb[0] : sb[1], 1);
+        double t1 = (b0 ? sb[3] : sb[2]) + __shfl_xor_sync(0xffffffffu, b0 ? sb[2] : sb[3], 1);
+        double s = (b1 ? t1 : t0) + __shfl_xor_sync(0xffffffffu, b1 ? t0 : t1, 2);
+        for (int o = 4; o < seg.len; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const int ks = (k + 32 * (lane & 3) + (lane & ~3)) / seg.len;
+        if ((lane & (seg.len - 1)) < 4 && ks < seg.n_seg)
+          seg.seg[((int64_t)i * seg.nj + j) * seg.n_seg + ks] = s;
       });
   double tot[1];
   if (block_reduce_last<1>(acc, 0u, a.part, a.ticket, tot) && threadIdx.x == 0) {
@@ -1134,31 +1073,54 @@ __global__ void __launch_bounds__(TB) fcg_update(TorsoArgs a) {
   }
 }
 
-// partial z.q (z in p1); last block: beta = -z.q / p.q
-__global__ void __launch_bounds__(TB) fcg_beta(TorsoArgs a) {
-  const float* __restrict__ z = a.p1;
+// partial z.q with z = M(r) formed on the fly (zero on air and at the pin,
+// where invd is zero); last block: beta = -z.q / p.q.  Forming z here and
+// again in fcg_p reads r and invd twice but saves its store and two loads and
+// the pass that made it (47 + 16 + 15 us on the full torso; 24 + 20 now).
+__global__ void __launch_bounds__(TB) fcg_beta(TorsoArgs a, pc::ZArgs z) {
+  if (a.iscal[IS_DONE]) return;
   const float* __restrict__ Ap = a.Ap;
+  const float* __restrict__ rv = a.r;
+  const float* __restrict__ invd = a.invd;
   double acc[1] = {0.0};
-  constexpr int LB = 8;
-  float zb[LB], qb[LB];
-  for_line_batches<LB>(
-      a, [&](int u, int64_t g) { zb[u] = z[g]; qb[u] = Ap[g]; },
-      [&](int u, int64_t) { acc[0] += (double)zb[u] * qb[u]; });
+  constexpr int LB = 4;
+  const int lane = threadIdx.x & 31;
+  float qb[LB], rb[LB], ib[LB];
+  for_aligned_lines<LB>(
+      a, [&](int u, int64_t g) { qb[u] = Ap[g]; rb[u] = rv[g]; ib[u] = invd[g]; },
+      [&](int u, int64_t, bool on) { if (!on) ib[u] = 0.0f; },
+      [&](int i, int j, int k) {
+#pragma unroll
+        for (int u = 0; u < LB; ++u)
+          if (ib[u] != 0.0f)
+            acc[0] += (double)pc::z_value(z, ib[u], rb[u], i, j, k + 32 * u + lane) * qb[u];
+      });
   double tot[1];
   if (block_reduce_last<1>(acc, 0u, a.part, a.ticket, tot) && threadIdx.x == 0)
     a.scal[SC_BETA] = -tot[0] / a.scal[SC_PAP];
 }
 
-// p = z + beta p
-__global__ void __launch_bounds__(TB) fcg_p(TorsoArgs a, int first) {
+// p = z + beta p, z = M(r) formed on the fly again
+__global__ void __launch_bounds__(TB) fcg_p(TorsoArgs a, pc::ZArgs z, int first) {
+  if (a.iscal[IS_DONE]) return;
   const float beta = first ? 0.0f : (float)a.scal[SC_BETA];
-  const float* __restrict__ z = a.p1;
+  const float* __restrict__ rv = a.r;
+  const float* __restrict__ invd = a.invd;
   float* __restrict__ p = a.p0;
-  constexpr int LB = 8;
-  float zb[LB], pb[LB];
-  for_line_batches<LB>(
-      a, [&](int u, int64_t g) { zb[u] = z[g]; pb[u] = p[g]; },
-      [&](int u, int64_t g) { p[g] = zb[u] + beta * pb[u]; });
+  constexpr int LB = 4;
+  const int lane = threadIdx.x & 31;
+  float pb[LB], rb[LB], ib[LB];
+  int64_t gb[LB];
+  for_aligned_lines<LB>(
+      a, [&](int u, int64_t g) { pb[u] = p[g]; rb[u] = rv[g]; ib[u] = invd[g]; },
+      [&](int u, int64_t g, bool on) { gb[u] = g; if (!on) ib[u] = 0.0f; },
+      [&](int i, int j, int k) {
+#pragma unroll
+        for (int u = 0; u < LB; ++u)
+          if (ib[u] != 0.0f)
+            p[gb[u]] = __fmaf_rn(beta, pb[u],
+                                 pc::z_value(z, ib[u], rb[u], i, j, k + 32 * u + lane));
+      });
 }
 
 __global__ void error_kernel(TorsoArgs a, const double* __restrict__ xstar, float* __restrict__ e) {
@@ -1189,12 +1151,14 @@ static hp_status fcg_graph(HpTorso* h, HpPrecond* p, int use_net, cudaStream_t s
   HP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   hp_status st = HP_OK;
   for (int it = 0; it < FCG_CHUNK && st == HP_OK; ++it) {
-    h->fspmv_fn<<<h->nblk_k[K_FCG_SPMV], TB, 0, s>>>(a);
-    fcg_update<<<h->nblk_k[K_FCG_UPDATE], TB, 0, s>>>(a);
-    st = pc::precond_apply(p, a.label, a.invd, a.r, a.p1, use_net > 0 && it % use_net == 0, s);
+    fcg_spmv<<<h->nblk_k[K_FCG_SPMV], TB, 0, s>>>(a, h->pcg);
+    fcg_update<<<h->nblk_k[K_FCG_UPDATE], TB, 0, s>>>(a, pc::precond_segments(p));
+    const int net = use_net > 0 && it % use_net == 0;
+    st = pc::precond_update(p, a.label, a.invd, a.r, net, s);
     if (st != HP_OK) break;
-    fcg_beta<<<h->nblk_k[K_FCG_BETA], TB, 0, s>>>(a);
-    fcg_p<<<h->nblk_k[K_FCG_P], TB, 0, s>>>(a, 0);
+    const pc::ZArgs z = pc::precond_z(p, net);
+    fcg_beta<<<h->nblk_k[K_FCG_BETA], TB, 0, s>>>(a, z);
+    fcg_p<<<h->nblk_k[K_FCG_P], TB, 0, s>>>(a, z, 0);
   }
   cudaError_t ce = cudaStreamEndCapture(s, &g);
   if (st != HP_OK) return st;
@@ -1203,17 +1167,6 @@ static hp_status fcg_graph(HpTorso* h, HpPrecond* p, int use_net, cudaStream_t s
   cudaGraphDestroy(g);
   h->fcg_graph_stream = s;
   h->fcg_graph_pc = serial;
-  return HP_OK;
-}
-
-// The flexible CG's own vectors, at its first solve.
-static hp_status fcg_vectors(HpTorso* h, cudaStream_t s) {
-  for (float** v : {&h->a.p0, &h->a.p1, &h->a.Ap}) {
-    if (*v) continue;
-    const hp_status st = tal(h, v, h->a.ng);
-    if (st != HP_OK) return st;
-    HP_CUDA_TRY(cudaMemsetAsync(*v, 0, h->a.ng * 4, s));
-  }
   return HP_OK;
 }
 
@@ -1246,17 +1199,18 @@ static hp_status fcg_run(HpTorso* h, HpPrecond* p, double tol, int fallback_iter
   // preconditioner's then only writes its own scratch and z)
   // z = M(r0), p = z (this first application also sets up anything the
   // preconditioner initialises lazily, before the capture)
-  st = pc::precond_apply(p, a.label, a.invd, a.r, a.p1, use_net, s);
+  const pc::ZArgs z0 = pc::precond_z(p, use_net);
+  st = pc::precond_begin(p, a.label, a.invd, a.r, use_net, s);
   if (st != HP_OK) return st;
-  fcg_p<<<h->nblk_k[K_FCG_P], TB, 0, s>>>(a, 1);
+  fcg_p<<<h->nblk_k[K_FCG_P], TB, 0, s>>>(a, z0, 1);
   st = fcg_graph(h, p, use_net, s);
   if (st != HP_OK) return st;
   bool restart = false;
   while (rel > tol) {
     if (restart) {
-      st = pc::precond_apply(p, a.label, a.invd, a.r, a.p1, use_net, s);
+      st = pc::precond_begin(p, a.label, a.invd, a.r, use_net, s);
       if (st != HP_OK) return st;
-      fcg_p<<<h->nblk_k[K_FCG_P], TB, 0, s>>>(a, 1);
+      fcg_p<<<h->nblk_k[K_FCG_P], TB, 0, s>>>(a, z0, 1);
       restart = false;
     }
     HP_CUDA_TRY(cudaGraphLaunch(h->fcg_graph[use_net == 0 ? 0 : (use_net == 1 ? 1 : (use_net == 2 ? 2 : 3))], s));
@@ -1344,6 +1298,7 @@ extern "C" hp_status hp_torso_solve_frame_fcg(HpTorso* h, HpPrecond* p, const fl
                         "the sharp-boundary operator; a smoothed-boundary (psi) handle solves "
                         "with hp_torso_solve_frame");
   HP_REQUIRE(p, "hp_torso_solve_frame_fcg: null preconditioner");
+  HP_REQUIRE(h->a.p0, "hp_torso_solve_frame_fcg: the torso's dims must be multiples of (8, 8, 256)");
   HP_REQUIRE(max_iter >= 1 && fallback_iter >= 1, "hp_torso_solve_frame_fcg: bad iteration limits");
   HP_REQUIRE(use_net == 0 || use_net == 1 || use_net == 2 || use_net == 4,
              "hp_torso_solve_frame_fcg: use_net must be 0, 1, 2 or 4");
@@ -1352,8 +1307,6 @@ extern "C" hp_status hp_torso_solve_frame_fcg(HpTorso* h, HpPrecond* p, const fl
   hp_status st = build_rhs(h, vm, vm_on_device, s);
   if (st != HP_OK) return st;
   hp_status result = HP_OK;
-  st = fcg_vectors(h, s);
-  if (st != HP_OK) return st;
   st = fcg_solve(h, p, tol, max_iter, fallback_iter, use_net, stats, &result, s);
   if (st != HP_OK) return st;
   st = readout(h, out, out_on_device, s);

@@ -95,3 +95,63 @@ def test_large_boxes_reach_the_true_residual(shape):
         np.testing.assert_array_equal(out, again)
     finally:
         solver.close()
+
+
+@pytest.mark.parametrize("agg", [-1, 4, 8, 16, 32, 64])
+def test_flexible_cg_takes_the_steps_of_a_host_loop(agg):
+    """The flexible CG forms z = M(r) inside its passes, from segment sums of
+    r; a host loop in FP64 around the preconditioner's own apply (z stored)
+    must take the same number of iterations for every aggregate edge."""
+    import torch
+    from tests.test_precond_gpu import _small, _wave_frames
+    from hrdayapy_b200.ecg.precond import LearnedPreconditioner
+    solver, grid, labels, table, dx, vox = _small(shape=(16, 24, 256))
+    pc = LearnedPreconditioner(solver, labels, len(table), coarse_agg=agg)
+    try:
+        vm = _wave_frames(vox, 3, 1)[1]
+        out, st = pc.solve_frame(vm, 1e-6, use_net=False)
+        assert st.status == 0 and st.rel_residual <= 1e-6 and st.restarts == 0
+        lab = torch.nn.functional.pad(torch.as_tensor(labels).long(), (1,) * 6).cuda()
+        sig = torch.as_tensor(table, dtype=torch.float64).cuda()[lab]
+        pin = int(pc.arrays.pin_cell)
+        faces = []
+        for ax in range(3):
+            a, b = sig.narrow(ax, 0, sig.shape[ax] - 1), sig.narrow(ax, 1, sig.shape[ax] - 1)
+            faces.append(torch.where((a > 0) & (b > 0), 2 * a * b / (a + b).clamp(min=1e-30), 0 * a)
+                         / (dx * 1e-3) ** 2)
+
+        def A(x):
+            y = torch.zeros_like(x)
+            for ax, w in enumerate(faces):
+                n = x.shape[ax]
+                f = w * (x.narrow(ax, 0, n - 1) - x.narrow(ax, 1, n - 1))
+                y.narrow(ax, 0, n - 1).add_(f)
+                y.narrow(ax, 1, n - 1).sub_(f)
+            y.view(-1)[pin] = 0.0
+            return y
+
+        def M(r):
+            r32 = r.float().contiguous()
+            z = torch.zeros_like(r32)
+            torch.cuda.synchronize()
+            pc.apply(r32.data_ptr(), z.data_ptr(), use_net=False)
+            torch.cuda.synchronize()
+            return z.double()
+
+        b = torch.zeros_like(sig)
+        b[lab > 0] = torch.as_tensor(solver.rhs(), dtype=torch.float64).cuda()
+        r, its = b.clone(), 0
+        z = M(r)
+        p = z.clone()
+        while torch.linalg.norm(r) >= 0.5e-6 * torch.linalg.norm(b) and its < 1000:
+            q = A(p)
+            pq = torch.sum(p * q)
+            r = r - torch.sum(p * r) / pq * q
+            z = M(r)
+            p = z - torch.sum(z * q) / pq * p
+            its += 1
+        # FP32 vectors against FP64 ones: a few per cent of the iterations
+        assert abs(its - st.iterations) <= 2 + 0.05 * its, (its, st.iterations)
+    finally:
+        pc.close()
+        solver.close()

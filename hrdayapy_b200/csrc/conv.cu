@@ -935,31 +935,58 @@ gsum_partial_kernel(const __nv_bfloat16* __restrict__ G, int64_t n, int coP, flo
   }
 }
 
-// gw[co][ci][t] and gb[co] from the partials, each summed in CTA order.
+// gw[co][ci][t] and gb[co] from the partials, each summed in CTA order.  A
+// warp's lanes take consecutive output channels of one (dz, M tile, dx, row),
+// so every read is a row segment of the partial tiles, RED_BATCH chunks in
+// flight (threads in gw's own order read one float a sector).  The bias blocks,
+// 16 channels each, bring their GS_BLOCKS rows to shared memory at once and add
+// them there.
+constexpr int RED_BATCH = 25;
 template <int CIN, int N>
 __global__ void __launch_bounds__(256)
 wgrad_reduce_kernel(const float* __restrict__ part, int nchunk, const float* __restrict__ gpart,
                     int cout, float* __restrict__ gw, float* __restrict__ gb) {
   using C = WgCfg<CIN, N>;
-  const int64_t nw = (int64_t)cout * CIN * 27;
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e < nw) {
-    const int t = (int)(e % 27), ci = (int)((e / 27) % CIN), co = (int)(e / (27 * CIN));
-    const int dzi = t / 9, dy = (t / 3) % 3, dx = t % 3;
-    const int slot = dy * C::G + ci / 8;
-    const int mt = slot / 16, row = (slot % 16) * 8 + ci % 8;
-    float s = 0.0f;
-    for (int c = 0; c < nchunk; ++c) {
-      const int64_t q = ((int64_t)dzi * nchunk + c) * (C::T * 3) + mt * 3 + dx;
-      s += part[(q * TILE_M + row) * N + co];
+  constexpr int ROWS = 8 * C::S;  // loaded rows over the M tiles
+  constexpr int W_BLOCKS = (9 * ROWS * N + 255) / 256;
+  if (blockIdx.x >= W_BLOCKS) {
+    __shared__ float sh[GS_BLOCKS][17];
+    const int c0 = (blockIdx.x - W_BLOCKS) * 16, c = threadIdx.x % 16;
+    float v[GS_BLOCKS / 16];
+#pragma unroll
+    for (int u = 0; u < GS_BLOCKS / 16; ++u)
+      v[u] = __ldg(gpart + (int64_t)(threadIdx.x / 16 + 16 * u) * N + c0 + c);
+#pragma unroll
+    for (int u = 0; u < GS_BLOCKS / 16; ++u) sh[threadIdx.x / 16 + 16 * u][c] = v[u];
+    __syncthreads();
+    if (threadIdx.x < 16 && c0 + c < cout) {
+      float s = 0.0f;
+#pragma unroll 16
+      for (int b = 0; b < GS_BLOCKS; ++b) s += sh[b][c];
+      gb[c0 + c] = s;
     }
-    gw[e] = s;
-  } else if (e < nw + cout) {
-    const int co = (int)(e - nw);
-    float s = 0.0f;
-    for (int b = 0; b < GS_BLOCKS; ++b) s += gpart[(int64_t)b * N + co];
-    gb[co] = s;
+    return;
   }
+  const int e = blockIdx.x * 256 + threadIdx.x;
+  const int co = e % N, slot_row = (e / N) % ROWS, q = e / (N * ROWS);  // q = 3 dz + dx
+  if (q >= 9 || co >= cout) return;
+  const int dzi = q / 3, dx = q % 3, slot = slot_row / 8;
+  const int dy = slot / C::G, ci = slot % C::G * 8 + slot_row % 8;
+  constexpr int64_t step = (int64_t)(C::T * 3) * TILE_M * N;
+  const float* src = part + (int64_t)dzi * nchunk * step +
+                     ((int64_t)(slot / 16 * 3 + dx) * TILE_M + slot % 16 * 8 + slot_row % 8) * N + co;
+  float s = 0.0f;
+  int k = 0;
+  for (; k + RED_BATCH <= nchunk; k += RED_BATCH) {
+    float v[RED_BATCH];
+#pragma unroll
+    for (int u = 0; u < RED_BATCH; ++u) v[u] = __ldg(src + (k + u) * step);
+#pragma unroll
+    for (int u = 0; u < RED_BATCH; ++u) s += v[u];
+  }
+#pragma unroll 4
+  for (; k < nchunk; ++k) s += __ldg(src + k * step);
+  gw[((int64_t)co * CIN + ci) * 27 + dzi * 9 + dy * 3 + dx] = s;
 }
 
 static int wg_chunks(int nl) {
@@ -1039,8 +1066,8 @@ hp_status wgrad3_launch(const void* X, const void* G, int D, int H, int W, int c
   gsum_partial_kernel<<<GS_BLOCKS, 256, 0, s>>>((const __nv_bfloat16*)G, (int64_t)D * H * W, N,
                                                 gpart);
   HP_CUDA_TRY(cudaGetLastError());
-  const int64_t nout = (int64_t)cout * cin * 27 + cout;
-  e->red<<<(unsigned)((nout + 255) / 256), 256, 0, s>>>(part, nchunk, gpart, cout, gw, gb);
+  const int red_blocks = (27 * cin * N + 255) / 256 + (cout + 15) / 16;  // weights, then biases
+  e->red<<<red_blocks, 256, 0, s>>>(part, nchunk, gpart, cout, gw, gb);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }

@@ -62,8 +62,18 @@ struct Dims {
 // Packs FP32 master weights w[co][ci][27] into the forward operand
 // [27][ci/8][coP][8] and the data-gradient operand [27][coP/8][ci][8]
 // (spatially flipped, channels transposed); padded channels are zero.
-__global__ void pack_kernel(const float* __restrict__ w, int cin, int cout,
-                            __nv_bfloat16* __restrict__ wp, __nv_bfloat16* __restrict__ wpt) {
+// One launch for all layers (blockIdx.y).
+struct PackArgs {
+  const float* w[NL];
+  __nv_bfloat16* wp[NL];
+  __nv_bfloat16* wpt[NL];
+  int cin[NL], cout[NL];
+};
+__global__ void pack_kernel(const __grid_constant__ PackArgs a) {
+  const int l = blockIdx.y, cin = a.cin[l], cout = a.cout[l];
+  const float* __restrict__ w = a.w[l];
+  __nv_bfloat16* __restrict__ wp = a.wp[l];
+  __nv_bfloat16* __restrict__ wpt = a.wpt[l];
   const int coP = padc(cout);
   const int64_t n = (int64_t)27 * cin * coP;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
@@ -102,50 +112,6 @@ __device__ __forceinline__ int64_t fine_of(const FeatArgs& a, int d, int h, int 
   return ((int64_t)fi * a.pj + fj) * a.pk + fk;
 }
 
-// raw[c] = mean over the 8 children of invd * r; partial sum of raw^2
-__global__ void __launch_bounds__(TB) feat_raw_kernel(FeatArgs a, float* __restrict__ raw,
-                                                     double* __restrict__ part) {
-  double acc = 0.0;
-  const int64_t n = a.c.n();
-  for (int64_t c = blockIdx.x * (int64_t)TB + threadIdx.x; c < n; c += (int64_t)gridDim.x * TB) {
-    const int w = c % a.c.W, h = (c / a.c.W) % a.c.H, d = (int)(c / ((int64_t)a.c.W * a.c.H));
-    float s = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int64_t g = fine_of(a, d, h, w, q);
-      if (a.label[g] != 0 && g != a.pin) s += a.invd[g] * a.r[g];
-    }
-    s *= 0.125f;
-    raw[c] = s;
-    acc += (double)s * s;
-  }
-  __shared__ double sh[TB];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = TB / 2; st > 0; st >>= 1) {
-    if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-// scale s = sqrt(mean raw^2) (single block), stored as float
-__global__ void scale_kernel(const double* part, int nparts, int64_t n, float* scale) {
-  __shared__ double sh[TB];
-  double a = 0.0;
-  for (int q = threadIdx.x; q < nparts; q += TB) a += part[q];
-  sh[threadIdx.x] = a;
-  __syncthreads();
-  for (int st = TB / 2; st > 0; st >>= 1) {
-    if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const double rms = sqrt(sh[0] / (double)(n > 0 ? n : 1));
-    scale[0] = (float)(rms > 1e-30 ? rms : 1e-30);
-  }
-}
-
 // feat[c][0] = raw / s, channels 1.. from the geometry tensor, channel 15
 // the coarse correction zh / s_z when there is a coarse level (zh != null)
 __global__ void feat_write_kernel(const float* __restrict__ raw, const __nv_bfloat16* __restrict__ geo,
@@ -165,95 +131,130 @@ __global__ void feat_write_kernel(const float* __restrict__ raw, const __nv_bflo
   }
 }
 
+// The pooling and upsampling passes below move eight channels (16 bytes) a
+// thread; sums are FP32 in child order.
+__device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
+  const __nv_bfloat162* b = (const __nv_bfloat162*)&u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float2 t = __bfloat1622float2(b[q]);
+    f[2 * q] = t.x;
+    f[2 * q + 1] = t.y;
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint4 u;
+  __nv_bfloat162* b = (__nv_bfloat162*)&u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    b[q] = __halves2bfloat162(__float2bfloat16(f[2 * q]), __float2bfloat16(f[2 * q + 1]));
+  return u;
+}
+// f where the stored activation a is positive, else 0 (ReLU backward)
+__device__ __forceinline__ uint4 masked8(const float (&f)[8], uint4 a) {
+  float v[8], g[8];
+  unpack8(a, v);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) g[q] = v[q] > 0.0f ? f[q] : 0.0f;
+  return pack8(g);
+}
+
 // 2 x 2 average pooling over (D, H): out dims (D/2, H/2, W)
 __global__ void pool_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
                             Dims o, int C) {
-  const int64_t n = o.n() * C;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int c = q % C;
-    const int64_t v = q / C;
-    const int w = v % o.W, h = (v / o.W) % o.H, d = (int)(v / ((int64_t)o.W * o.H));
-    const int Hi = 2 * o.H;
-    float s = 0.0f;
+  const int C8 = C / 8, n = (int)o.n() * C8;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int c = q % C8, v = q / C8;
+    const int w = v % o.W, h = (v / o.W) % o.H, d = v / (o.W * o.H);
+    uint4 u[4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int k = 0; k < 4; ++k)
+      u[k] = *(const uint4*)(in + ((((int64_t)(2 * d + (k >> 1)) * 2 * o.H + 2 * h + (k & 1)) * o.W) +
+                                   w) * C + 8 * c);
+    float s[8] = {};
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
-        s += __bfloat162float(in[((((int64_t)(2 * d + a) * Hi + 2 * h + b) * o.W) + w) * C + c]);
-    out[q] = __float2bfloat16(0.25f * s);
+    for (int k = 0; k < 4; ++k) {
+      float f[8];
+      unpack8(u[k], f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] += f[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] *= 0.25f;
+    *(uint4*)(out + (int64_t)v * C + 8 * c) = pack8(s);
   }
 }
 
-// backward of pooling: gin (fine) += 0.25 * gout (coarse)
+// backward of pooling and of the ReLU before it: gin (fine) += 0.25 * gout
+// (coarse), rounded, then zero where the activation is not positive
 __global__ void pool_back_kernel(const __nv_bfloat16* __restrict__ gout, __nv_bfloat16* __restrict__ gin,
-                                 Dims f, int C) {
-  const int64_t n = f.n() * C;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int c = q % C;
-    const int64_t v = q / C;
-    const int w = v % f.W, h = (v / f.W) % f.H, d = (int)(v / ((int64_t)f.W * f.H));
+                                 const __nv_bfloat16* __restrict__ act, Dims f, int C) {
+  const int C8 = C / 8, n = (int)f.n() * C8;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int c = q % C8, v = q / C8;
+    const int w = v % f.W, h = (v / f.W) % f.H, d = v / (f.W * f.H);
     const int64_t vc = ((int64_t)(d / 2) * (f.H / 2) + h / 2) * f.W + w;
-    gin[q] = __float2bfloat16(__bfloat162float(gin[q]) + 0.25f * __bfloat162float(gout[vc * C + c]));
+    const uint4 u = *(const uint4*)(gin + 8 * (int64_t)q);
+    const uint4 t = *(const uint4*)(gout + vc * C + 8 * c);
+    const uint4 a = *(const uint4*)(act + 8 * (int64_t)q);
+    float g[8], o[8];
+    unpack8(u, g);
+    unpack8(t, o);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) g[e] += 0.25f * o[e];
+    *(uint4*)(gin + 8 * (int64_t)q) = masked8(g, a);
   }
 }
 
 // out (fine, C1 + C2 channels) = [nearest-upsampled coarse (C1) | skip (C2)]
 __global__ void upcat_kernel(const __nv_bfloat16* __restrict__ coarse, const __nv_bfloat16* __restrict__ skip,
                              __nv_bfloat16* __restrict__ out, Dims f, int C1, int C2) {
-  const int C = C1 + C2;
-  const int64_t n = f.n() * (C / 8);
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int g = q % (C / 8);
-    const int64_t v = q / (C / 8);
-    const int w = v % f.W, h = (v / f.W) % f.H, d = (int)(v / ((int64_t)f.W * f.H));
+  const int C = C1 + C2, C8 = C / 8, n = (int)f.n() * C8;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int g = q % C8, v = q / C8;
     uint4 val;
     if (g * 8 < C1) {
+      const int w = v % f.W, h = (v / f.W) % f.H, d = v / (f.W * f.H);
       const int64_t vc = ((int64_t)(d / 2) * (f.H / 2) + h / 2) * f.W + w;
       val = *(const uint4*)(coarse + vc * C1 + g * 8);
     } else {
-      val = *(const uint4*)(skip + v * C2 + (g * 8 - C1));
+      val = *(const uint4*)(skip + (int64_t)v * C2 + (g * 8 - C1));
     }
-    *(uint4*)(out + v * C + g * 8) = val;
+    *(uint4*)(out + 8 * (int64_t)q) = val;
   }
 }
 
-// backward of upcat: gcoarse = sum of the 4 fine children's first C1
-// channels, gskip = remaining channels (overwrites both)
+// backward of upcat: gcoarse = sum of the 4 fine children's first C1 channels,
+// zero where the coarse activation is not positive (the ReLU before the
+// upsampling); gskip = the remaining channels (overwrites both)
 __global__ void upcat_back_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ gcoarse,
-                                  __nv_bfloat16* __restrict__ gskip, Dims f, int C1, int C2) {
-  const int C = C1 + C2;
-  const Dims c{f.D / 2, f.H / 2, f.W};
-  const int64_t nc = c.n() * C1;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nc;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int ch = q % C1;
-    const int64_t v = q / C1;
-    const int w = v % c.W, h = (v / c.W) % c.H, d = (int)(v / ((int64_t)c.W * c.H));
-    float s = 0.0f;
+                                  const __nv_bfloat16* __restrict__ act, __nv_bfloat16* __restrict__ gskip,
+                                  Dims f, int C1, int C2) {
+  const int C = C1 + C2, H = f.H / 2;
+  const int nc = (int)(f.n() / 4) * (C1 / 8), nf = (int)f.n() * (C2 / 8);
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nc + nf; q += gridDim.x * blockDim.x) {
+    if (q < nc) {
+      const int ch = q % (C1 / 8), v = q / (C1 / 8);
+      const int w = v % f.W, h = (v / f.W) % H, d = v / (f.W * H);
+      uint4 u[4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+      for (int k = 0; k < 4; ++k)
+        u[k] = *(const uint4*)(gu + ((((int64_t)(2 * d + (k >> 1)) * f.H + 2 * h + (k & 1)) * f.W) +
+                                     w) * C + 8 * ch);
+      float s[8] = {};
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
-        s += __bfloat162float(gu[((((int64_t)(2 * d + a) * f.H + 2 * h + b) * f.W) + w) * C + ch]);
-    gcoarse[q] = __float2bfloat16(s);
+      for (int k = 0; k < 4; ++k) {
+        float t[8];
+        unpack8(u[k], t);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += t[e];
+      }
+      *(uint4*)(gcoarse + 8 * (int64_t)q) = masked8(s, *(const uint4*)(act + 8 * (int64_t)q));
+    } else {
+      const int e = q - nc, ch = e % (C2 / 8), v = e / (C2 / 8);
+      *(uint4*)(gskip + 8 * (int64_t)e) = *(const uint4*)(gu + (int64_t)v * C + C1 + 8 * ch);
+    }
   }
-  const int64_t nf = f.n() * C2;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nf;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int ch = q % C2;
-    const int64_t v = q / C2;
-    gskip[q] = gu[v * C + C1 + ch];
-  }
-}
-
-// g = g * (a > 0) (ReLU backward on a stored activation)
-__global__ void relu_mask_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ a, int64_t n) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
-       q += (int64_t)gridDim.x * blockDim.x)
-    if (!(__bfloat162float(a[q]) > 0.0f)) g[q] = __float2bfloat16(0.0f);
 }
 
 // Coarse level: per aggregate the sum of r over its active, unpinned cells.
@@ -269,12 +270,6 @@ struct CoarseArgs {
   float* zbox;            // zc by box
 };
 
-// aggregate edge lengths are powers of two: shifts instead of divisions
-__device__ __forceinline__ int coarse_of(const CoarseArgs& c, int i, int j, int k) {
-  const int sh = c.ag_shift;
-  return c.box2c[((i >> sh) * c.nbj + (j >> sh)) * c.nbk + (k >> sh)];
-}
-
 __global__ void __launch_bounds__(TB) coarse_restrict_kernel(CoarseArgs c, const float* __restrict__ r) {
   const int I = blockIdx.x;
   const int b = c.c_box[I];
@@ -282,12 +277,23 @@ __global__ void __launch_bounds__(TB) coarse_restrict_kernel(CoarseArgs c, const
   const int sh = c.ag_shift, m = c.ag - 1;
   const int n = 1 << (3 * sh);
   double acc = 0.0;
-  for (int t = threadIdx.x; t < n; t += TB) {
-    const int i = (bi << sh) + (t >> (2 * sh)), j = (bj << sh) + ((t >> sh) & m),
-              k = (bk << sh) + (t & m);
-    if (i >= c.ni || j >= c.nj || k >= c.nk) continue;
-    const int64_t g = ((int64_t)(i + 1) * c.pj + (j + 1)) * c.pk + (k + 1);
-    if (c.label[g] != 0 && g != c.pin) acc += (double)r[g];
+  constexpr int B = 8;  // cells in flight a thread
+  for (int t0 = threadIdx.x; t0 < n; t0 += TB * B) {
+    float v[B];
+    bool on[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int t = t0 + TB * u;
+      const int i = (bi << sh) + (t >> (2 * sh)), j = (bj << sh) + ((t >> sh) & m),
+                k = (bk << sh) + (t & m);
+      on[u] = t < n && i < c.ni && j < c.nj && k < c.nk;
+      const int64_t g = on[u] ? ((int64_t)(i + 1) * c.pj + (j + 1)) * c.pk + (k + 1) : 0;
+      on[u] = on[u] && c.label[g] != 0 && g != c.pin;
+      v[u] = r[g];
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+      if (on[u]) acc += (double)v[u];
   }
   __shared__ double red[TB];
   red[threadIdx.x] = acc;
@@ -356,61 +362,126 @@ __global__ void __launch_bounds__(TB) coarse_matvec_kernel(CoarseArgs c) {
   }
 }
 
-// zh[c] = coarse correction of the aggregate holding network cell c (its 8
-// fine children share one aggregate, ag being even); partial sums of zh^2
-__global__ void __launch_bounds__(TB) coarse_feat_kernel(CoarseArgs c, Dims cd, float* __restrict__ zh,
-                                                         double* __restrict__ part) {
-  double acc = 0.0;
-  const int64_t n = cd.n();
-  for (int64_t q = blockIdx.x * (int64_t)TB + threadIdx.x; q < n; q += (int64_t)gridDim.x * TB) {
-    const int w = q % cd.W, h = (q / cd.W) % cd.H, d = (int)(q / ((int64_t)cd.W * cd.H));
-    const int I = coarse_of(c, 2 * d, 2 * h, 2 * w);
-    const float v = I >= 0 ? c.zc[I] : 0.0f;
-    zh[q] = v;
-    acc += (double)v * v;
+// raw[c] = mean over the 8 children of invd * r (0 on air and at the pin) and
+// zh[c] = coarse correction of the aggregate holding network
+// cell c (its 8 fine children share one aggregate, ag being even; null
+// without a coarse level).  The last block turns the sums of squares into the
+// scales: scale[0] = RMS of raw, [1] = RMS of zh, [2] = the output's (that of
+// zh where there is a coarse level, else that of raw).
+__global__ void __launch_bounds__(TB) feat_raw_kernel(FeatArgs a, CoarseArgs cc,
+                                                     float* __restrict__ raw,
+                                                     float* __restrict__ zh,
+                                                     double* __restrict__ part,
+                                                     unsigned int* ticket, float* scale) {
+  double acc[2] = {0.0, 0.0};
+  const int n = (int)a.c.n();
+  for (int c = blockIdx.x * TB + threadIdx.x; c < n; c += gridDim.x * TB) {
+    const int w = c % a.c.W, h = (c / a.c.W) % a.c.H, d = c / (a.c.W * a.c.H);
+    float iv[8], rv[8];
+    bool on[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int64_t g = fine_of(a, d, h, w, q);
+      on[q] = a.label[g] != 0 && g != a.pin;
+      iv[q] = a.invd[g];
+      rv[q] = a.r[g];
+    }
+    float s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (on[q]) s += iv[q] * rv[q];
+    s *= 0.125f;
+    raw[c] = s;
+    acc[0] += (double)s * s;
+    if (zh) {
+      const float v = cc.zbox[((2 * d >> cc.ag_shift) * cc.nbj + (2 * h >> cc.ag_shift)) * cc.nbk +
+                              (2 * w >> cc.ag_shift)];
+      zh[c] = v;
+      acc[1] += (double)v * v;
+    }
   }
-  __shared__ double sh[TB];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = TB / 2; st > 0; st >>= 1) {
-    if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
+  __shared__ double sh[2][TB];
+  __shared__ bool last;
+  auto over_block = [&]() {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) sh[k][threadIdx.x] = acc[k];
     __syncthreads();
+    for (int st = TB / 2; st > 0; st >>= 1) {
+      if ((int)threadIdx.x < st)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + st];
+      __syncthreads();
+    }
+  };
+  over_block();
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = sh[0][0];
+    part[2 * blockIdx.x + 1] = sh[1][0];
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  acc[0] = acc[1] = 0.0;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += TB) {
+    acc[0] += __ldcg(part + 2 * q);
+    acc[1] += __ldcg(part + 2 * q + 1);
+  }
+  over_block();
+  if (threadIdx.x == 0) {
+    *ticket = 0u;
+    float sc[2];
+    for (int k = 0; k < 2; ++k) {
+      const double rms = sqrt(sh[k][0] / (double)(n > 0 ? n : 1));
+      sc[k] = (float)(rms > 1e-30 ? rms : 1e-30);
+    }
+    scale[0] = sc[0];
+    scale[1] = sc[1];
+    scale[2] = zh ? sc[1] : sc[0];
+  }
 }
 
 struct ProlongArgs {
-  CoarseArgs c;
   int pj, pk;
   int64_t ng, pin;
   const uint8_t* label;
   const float* invd;
   const float* r;
-  const float* y;       // coarse FP32 output
-  const float* scale;
-  float omega;
-  Dims cd;
-  int use_net;
 };
 
 // z = omega * invd * r + s * y[parent] + zc[aggregate] on active fine cells
-// (0 elsewhere); one block per padded (i, j) row, threads along k, so the
-// coordinates come from the launch shape instead of divisions.
-__global__ void __launch_bounds__(TB) prolong_kernel(ProlongArgs a, float* __restrict__ z) {
-  const float s = a.use_net ? a.scale[2] : 0.0f;
-  const int i = blockIdx.y, j = blockIdx.x;
-  const int64_t row = ((int64_t)i * a.pj + j) * a.pk;
-  const bool inner = i > 0 && j > 0 && j < a.pj - 1 && i < (int)(a.ng / ((int64_t)a.pj * a.pk)) - 1;
-  for (int k = threadIdx.x; k < a.pk; k += TB) {
-    const int64_t g = row + k;
-    float v = 0.0f;
-    if (inner && a.label[g] != 0 && g != a.pin) {
-      v = a.omega * a.invd[g] * a.r[g];
-      const int ui = i - 1, uj = j - 1, uk = k - 1;
-      if (a.use_net) v += s * a.y[((int64_t)(ui >> 1) * a.cd.H + (uj >> 1)) * a.cd.W + (uk >> 1)];
-      if (a.c.nc > 0) v += a.c.zc[coarse_of(a.c, ui, uj, uk)];
+// (0 elsewhere), in z_value's order and rounding; one warp per padded (i, j)
+// row, four steps of 32 cells in flight.  (A block per row, its second step
+// two cells wide, took 24 us on 128 x 112 x 256 and 47 us on 192 x 160 x 256.)
+__global__ void __launch_bounds__(TB) prolong_kernel(ProlongArgs a, ZArgs zv, float* __restrict__ z) {
+  const int lane = threadIdx.x & 31, n_rows = (int)(a.ng / a.pk);
+  const int row = blockIdx.x * (TB / 32) + (threadIdx.x >> 5);
+  if (row >= n_rows) return;
+  const int i = row / a.pj - 1, j = row % a.pj - 1;
+  const int64_t base = (int64_t)row * a.pk;
+  const bool inner = i >= 0 && j >= 0 && j < a.pj - 2 && i < n_rows / a.pj - 2;
+  constexpr int B = 4;
+  for (int k0 = lane; k0 < a.pk; k0 += 32 * B) {
+    uint8_t lab[B];
+    float iv[B], rv[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int k = k0 + 32 * u;
+      lab[u] = 0;
+      if (inner && k < a.pk) {
+        lab[u] = a.label[base + k];
+        iv[u] = a.invd[base + k];
+        rv[u] = a.r[base + k];
+      }
     }
-    z[g] = v;
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int k = k0 + 32 * u;
+      if (k < a.pk)
+        z[base + k] =
+            lab[u] != 0 && base + k != a.pin ? z_value(zv, iv[u], rv[u], i, j, k - 1) : 0.0f;
+    }
   }
 }
 
@@ -568,7 +639,10 @@ struct HpPrecond {
   // gradients
   __nv_bfloat16 *gout, *g_d1b, *g_d1a, *g_u1, *g_d2b, *g_e1b, *g_d2a, *g_u2, *g_e3b, *g_e2b,
       *g_e3a, *g_p2, *g_e2a, *g_p1, *g_e1a;
+  cudaStream_t side;         // weight gradients
+  cudaEvent_t fork, join;
   double* part;
+  unsigned int* ticket;
   double* dots;              // r.z, z.A z, r.e of the energy loss
   double* loss;
   float* zbuf;               // M(r) on the fine grid (training)
@@ -614,9 +688,15 @@ extern "C" hp_status hp_precond_destroy(HpPrecond* h);
   } while (0)
 
 static hp_status repack(HpPrecond* h, cudaStream_t s) {
+  PackArgs a;
   for (int l = 0; l < NL; ++l) {
-    pack_kernel<<<256, 256, 0, s>>>(h->par + h->off_w[l], LCIN[l], LCOUT[l], h->wp[l], h->wpt[l]);
+    a.w[l] = h->par + h->off_w[l];
+    a.wp[l] = h->wp[l];
+    a.wpt[l] = h->wpt[l];
+    a.cin[l] = LCIN[l];
+    a.cout[l] = LCOUT[l];
   }
+  pack_kernel<<<dim3(54, NL), 256, 0, s>>>(a);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
@@ -775,6 +855,8 @@ extern "C" hp_status hp_precond_create(const HpPrecondDesc* d, HpPrecond** out, 
   h->L[2] = Dims{d->ni / 4, d->nj / 4, d->nk / 2};
   h->L[3] = Dims{d->ni / 8, d->nj / 8, d->nk / 2};
   h->step = 0;
+  h->side = nullptr;
+  h->fork = h->join = nullptr;
   int nsm = 148;
   {
     int dev = 0;
@@ -791,6 +873,17 @@ extern "C" hp_status hp_precond_create(const HpPrecondDesc* d, HpPrecond** out, 
     o += LCOUT[l];
   }
   h->n_par = o;
+  {
+    const cudaError_t e1 = cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking);
+    const cudaError_t e2 = cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming);
+    const cudaError_t e3 = cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming);
+    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
+      hp_precond_destroy(h);
+      hp::set_error("hp_precond_create: no stream or event: %s",
+                    cudaGetErrorString(e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3)));
+      return HP_ERR_CUDA;
+    }
+  }
   PC_TRY(pal(h, &h->par, o));
   PC_TRY(pal(h, &h->grad, o));
   PC_TRY(pal(h, &h->adam_m, o));
@@ -866,6 +959,8 @@ extern "C" hp_status hp_precond_create(const HpPrecondDesc* d, HpPrecond** out, 
   PC_TRY(pal(h, &h->g_p1, n2 * 16));
   PC_TRY(pal(h, &h->g_e1a, n1 * 16));
   PC_TRY(pal(h, &h->part, 3 * h->nblk));
+  PC_TRY(pal(h, &h->ticket, 1));
+  HP_CUDA_TRY(cudaMemsetAsync(h->ticket, 0, 4, s));
   PC_TRY(pal(h, &h->dots, 3));
   PC_TRY(pal(h, &h->zbuf, h->ng));
   PC_TRY(pal(h, &h->az, h->ng));
@@ -968,17 +1063,10 @@ hp_status precond_forward(HpPrecond* h, const uint8_t* label, const float* invd,
                           cudaStream_t s) {
   FeatArgs fa{h->pj, h->pk, h->pin, label, invd, r, h->L[1]};
   const int64_t n1 = h->L[1].n();
-  feat_raw_kernel<<<h->nblk, TB, 0, s>>>(fa, h->raw, h->part);
-  scale_kernel<<<1, TB, 0, s>>>(h->part, h->nblk, n1, h->scale);
-  if (h->nc > 0) {
-    // the network also sees the coarse correction; its output is scaled like
-    // that field (the error it refines), else like the input
-    coarse_feat_kernel<<<h->nblk, TB, 0, s>>>(coarse_args(h, label), h->L[1], h->zh, h->part);
-    scale_kernel<<<1, TB, 0, s>>>(h->part, h->nblk, n1, h->scale + 1);
-    HP_CUDA_TRY(cudaMemcpyAsync(h->scale + 2, h->scale + 1, 4, cudaMemcpyDeviceToDevice, s));
-  } else {
-    HP_CUDA_TRY(cudaMemcpyAsync(h->scale + 2, h->scale, 4, cudaMemcpyDeviceToDevice, s));
-  }
+  // the network also sees the coarse correction; its output is scaled like
+  // that field (the error it refines), else like the input
+  feat_raw_kernel<<<(int)std::min<int64_t>(h->nblk, (n1 + TB - 1) / TB), TB, 0, s>>>(
+      fa, coarse_args(h, label), h->raw, h->nc > 0 ? h->zh : nullptr, h->part, h->ticket, h->scale);
   feat_write_kernel<<<grid_for(n1), 256, 0, s>>>(h->raw, h->geo, h->scale, h->feat, n1,
                                                  h->nc > 0 ? h->zh : nullptr);
   HP_CUDA_TRY(cudaGetLastError());
@@ -986,10 +1074,10 @@ hp_status precond_forward(HpPrecond* h, const uint8_t* label, const float* invd,
 #define FW(x) do { st = (x); if (st != HP_OK) return st; } while (0)
   FW(conv(h, E1A, h->feat, h->e1a, tc::EPI_RELU, nullptr, s));
   FW(conv(h, E1B, h->e1a, h->e1b, tc::EPI_RELU, nullptr, s));
-  pool_kernel<<<grid_for(h->L[2].n() * 16), 256, 0, s>>>(h->e1b, h->p1, h->L[2], 16);
+  pool_kernel<<<grid_for(h->L[2].n() * 2), 256, 0, s>>>(h->e1b, h->p1, h->L[2], 16);
   FW(conv(h, E2A, h->p1, h->e2a, tc::EPI_RELU, nullptr, s));
   FW(conv(h, E2B, h->e2a, h->e2b, tc::EPI_RELU, nullptr, s));
-  pool_kernel<<<grid_for(h->L[3].n() * 32), 256, 0, s>>>(h->e2b, h->p2, h->L[3], 32);
+  pool_kernel<<<grid_for(h->L[3].n() * 4), 256, 0, s>>>(h->e2b, h->p2, h->L[3], 32);
   FW(conv(h, E3A, h->p2, h->e3a, tc::EPI_RELU, nullptr, s));
   FW(conv(h, E3B, h->e3a, h->e3b, tc::EPI_RELU, nullptr, s));
   upcat_kernel<<<grid_for(h->L[2].n() * 12), 256, 0, s>>>(h->e3b, h->e2b, h->u2, h->L[2], 64, 32);
@@ -1035,13 +1123,19 @@ hp_status precond_begin(HpPrecond* h, const uint8_t* label, const float* invd, c
   return precond_forward(h, label, invd, r, s);
 }
 
+// z = M(r) from the coarse solve's and the network's results.
+static void prolong(HpPrecond* h, const uint8_t* label, const float* invd, const float* r, float* z,
+                    int use_net, cudaStream_t s) {
+  const ProlongArgs pa{h->pj, h->pk, h->ng, h->pin, label, invd, r};
+  const int rows = (int)(h->ng / h->pk);
+  prolong_kernel<<<(rows + TB / 32 - 1) / (TB / 32), TB, 0, s>>>(pa, precond_z(h, use_net), z);
+}
+
 static hp_status precond_apply(HpPrecond* h, const uint8_t* label, const float* invd,
                                const float* r, float* z, int use_net, cudaStream_t s) {
   const hp_status st = precond_begin(h, label, invd, r, use_net, s);
   if (st != HP_OK) return st;
-  ProlongArgs pa{coarse_args(h, label), h->pj, h->pk, h->ng, h->pin, label, invd, r, h->y,
-                 h->scale, h->omega, h->L[1], use_net};
-  prolong_kernel<<<dim3(h->pj, (unsigned)(h->ng / ((int64_t)h->pj * h->pk))), TB, 0, s>>>(pa, z);
+  prolong(h, label, invd, r, z, use_net, s);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
@@ -1066,15 +1160,21 @@ extern "C" hp_status hp_precond_train_step(HpPrecond* h, const uint8_t* label, c
   if (st != HP_OK) return st;
   const Dims L1 = h->L[1], L2 = h->L[2], L3 = h->L[3];
   const int64_t n1 = L1.n(), n2 = L2.n(), n3 = L3.n();
-  ProlongArgs pa{coarse_args(h, label), h->pj, h->pk, h->ng, h->pin, label, invd, r, h->y,
-                 h->scale, h->omega, h->L[1], 1};
-  prolong_kernel<<<dim3(h->pj, (unsigned)(h->ng / ((int64_t)h->pj * h->pk))), TB, 0, s>>>(pa, h->zbuf);
+  hp::pc::prolong(h, label, invd, r, h->zbuf, 1, s);
   EnergyArgs ea{h->pj, h->pk, h->ng, h->pin, label, h->T32, r, e, h->zbuf, h->az};
   energy_dots_kernel<<<h->nblk, TB, 0, s>>>(ea, h->part);
   sum3_kernel<<<1, TB, 0, s>>>(h->part, h->nblk, h->dots);
   energy_grad_kernel<<<h->nblk, TB, 0, s>>>(ea, L1, h->dots, h->scale, h->gout, h->loss);
-  HP_CUDA_TRY(cudaMemsetAsync(h->grad, 0, h->n_par * 4, s));
-#define BW(x) do { st = (x); if (st != HP_OK) return st; } while (0)
+  // a layer's weight gradient hangs on its output gradient alone: the side
+  // stream takes it beside the chain of data gradients (no buffer it reads is
+  // written again in this step), and joins before the update
+  auto wgrad = [&](HpPrecond* hh, int l, const __nv_bfloat16* X, const __nv_bfloat16* G,
+                   cudaStream_t ss) -> hp_status {
+    HP_CUDA_TRY(cudaEventRecord(hh->fork, ss));
+    HP_CUDA_TRY(cudaStreamWaitEvent(hh->side, hh->fork, 0));
+    return hp::pc::wgrad(hh, l, X, G, hh->side);
+  };
+#define BW(x) do { st = (x); if (st != HP_OK) { cudaStreamSynchronize(h->side); return st; } } while (0)
   // OUT (linear, 16 -> 1 padded to 16)
   BW(wgrad(h, OUT, h->d1b, h->gout, s));
   BW(dgrad(h, OUT, h->gout, h->g_d1b, h->d1b, s));          // -> dpre of D1B
@@ -1082,30 +1182,30 @@ extern "C" hp_status hp_precond_train_step(HpPrecond* h, const uint8_t* label, c
   BW(dgrad(h, D1B, h->g_d1b, h->g_d1a, h->d1a, s));         // -> dpre of D1A
   BW(wgrad(h, D1A, h->u1, h->g_d1a, s));
   BW(dgrad(h, D1A, h->g_d1a, h->g_u1, nullptr, s));         // d u1 (48)
-  upcat_back_kernel<<<grid_for(n1 * 16), 256, 0, s>>>(h->g_u1, h->g_d2b, h->g_e1b, L1, 32, 16);
-  relu_mask_kernel<<<grid_for(n2 * 32), 256, 0, s>>>(h->g_d2b, h->d2b, n2 * 32);
+  upcat_back_kernel<<<grid_for(n2 * 4 + n1 * 2), 256, 0, s>>>(h->g_u1, h->g_d2b, h->d2b, h->g_e1b,
+                                                               L1, 32, 16);
   BW(wgrad(h, D2B, h->d2a, h->g_d2b, s));
   BW(dgrad(h, D2B, h->g_d2b, h->g_d2a, h->d2a, s));
   BW(wgrad(h, D2A, h->u2, h->g_d2a, s));
   BW(dgrad(h, D2A, h->g_d2a, h->g_u2, nullptr, s));         // d u2 (96)
-  upcat_back_kernel<<<grid_for(n2 * 64), 256, 0, s>>>(h->g_u2, h->g_e3b, h->g_e2b, L2, 64, 32);
-  relu_mask_kernel<<<grid_for(n3 * 64), 256, 0, s>>>(h->g_e3b, h->e3b, n3 * 64);
+  upcat_back_kernel<<<grid_for(n3 * 8 + n2 * 4), 256, 0, s>>>(h->g_u2, h->g_e3b, h->e3b, h->g_e2b,
+                                                               L2, 64, 32);
   BW(wgrad(h, E3B, h->e3a, h->g_e3b, s));
   BW(dgrad(h, E3B, h->g_e3b, h->g_e3a, h->e3a, s));
   BW(wgrad(h, E3A, h->p2, h->g_e3a, s));
   BW(dgrad(h, E3A, h->g_e3a, h->g_p2, nullptr, s));
-  pool_back_kernel<<<grid_for(n2 * 32), 256, 0, s>>>(h->g_p2, h->g_e2b, L2, 32);
-  relu_mask_kernel<<<grid_for(n2 * 32), 256, 0, s>>>(h->g_e2b, h->e2b, n2 * 32);
+  pool_back_kernel<<<grid_for(n2 * 4), 256, 0, s>>>(h->g_p2, h->g_e2b, h->e2b, L2, 32);
   BW(wgrad(h, E2B, h->e2a, h->g_e2b, s));
   BW(dgrad(h, E2B, h->g_e2b, h->g_e2a, h->e2a, s));
   BW(wgrad(h, E2A, h->p1, h->g_e2a, s));
   BW(dgrad(h, E2A, h->g_e2a, h->g_p1, nullptr, s));
-  pool_back_kernel<<<grid_for(n1 * 16), 256, 0, s>>>(h->g_p1, h->g_e1b, L1, 16);
-  relu_mask_kernel<<<grid_for(n1 * 16), 256, 0, s>>>(h->g_e1b, h->e1b, n1 * 16);
+  pool_back_kernel<<<grid_for(n1 * 2), 256, 0, s>>>(h->g_p1, h->g_e1b, h->e1b, L1, 16);
   BW(wgrad(h, E1B, h->e1a, h->g_e1b, s));
   BW(dgrad(h, E1B, h->g_e1b, h->g_e1a, h->e1a, s));
   BW(wgrad(h, E1A, h->feat, h->g_e1a, s));
 #undef BW
+  HP_CUDA_TRY(cudaEventRecord(h->join, h->side));
+  HP_CUDA_TRY(cudaStreamWaitEvent(s, h->join, 0));
   HP_CUDA_TRY(cudaGetLastError());
   if (lr > 0.0f) {
     h->step += 1;
@@ -1164,6 +1264,9 @@ extern "C" hp_status hp_precond_coarse_info(const HpPrecond* h, int32_t* agg, in
 extern "C" hp_status hp_precond_destroy(HpPrecond* h) {
   if (!h) return HP_OK;
   for (void* p : h->allocs) cudaFree(p);
+  if (h->side) cudaStreamDestroy(h->side);
+  if (h->fork) cudaEventDestroy(h->fork);
+  if (h->join) cudaEventDestroy(h->join);
   delete h;
   return HP_OK;
 }

@@ -93,8 +93,10 @@ struct MonoArgs {
   // at n_active_pad (n_active rounded up to a warp); slot >> bv_shift = brick
   int32_t n_active, n_active_pad, bv_shift;
   const int32_t* active_slot;
-  // theta-scheme: the CG solution x ([slots | Purkinje]) of the step
+  // theta-scheme: the CG solution x + pend p ([slots | Purkinje]) of the step
   const float* cn_x;
+  const float* cn_p;
+  const double* cn_pend;
 };
 
 // TTP06 phenotype table (ttp06_phenotype_constants.py:54-61), index = pheno-1.
@@ -687,13 +689,20 @@ mono_pipe_kernel(MonoArgs a, int step_off) {
 // dot products are FP64 with deterministic last-block grid reductions.  The
 // warm-start residual rhs - M W equals Lh W, so one stencil pass gives the
 // initial residual, the norm of the right-hand side and the first direction.
+// An iteration is one stencil pass and one vector pass: with <p, q>_w the
+// stencil pass sums ||r||^2, <r, z>_w, <r, q>, <q, q>, <r, D^-1 q>_w and <q,
+// D^-1 q>_w, which predict the next residual's norms, hence beta and the
+// stopping test; the vector pass then updates x, r and p together.  The last
+// iteration's step is left pending (CN_PEND) for the kernel that clamps x.
+// (Separate x / r and p passes, the norms from the former, moved 56 bytes an
+// entry and iteration against 44 here, and twice the launches.)
 // Every iteration kernel returns at once when the done flag is set, so the
 // host may enqueue iterations in chunks and test the flag between chunks.
-enum CnScal : int { CN_BB = 0, CN_RZ, CN_PQ, CN_ALPHA, CN_BETA, CN_RR, N_CN_SCAL };
+enum CnScal : int { CN_BB = 0, CN_ALPHA, CN_BETA, CN_PEND, CN_RR, N_CN_SCAL };
 enum CnIScal : int { CI_DONE = 0, CI_ITER, CI_TOTAL, CI_SOLVES, CI_UNCONV, CI_BREAK, CI_LOOP,
                      N_CN_ISCAL };
 constexpr int CN_TB = 256;   // threads of the vector kernels
-constexpr int CN_NPART = 4;  // partials per block
+constexpr int CN_NPART = 8;  // partials per block
 
 struct CnArgs {
   int64_t n;             // n_slots + n_pk
@@ -718,7 +727,7 @@ struct CnArgs {
 template <int NT, int NV>
 __device__ bool cn_reduce_last(double (&v)[NV], const CnArgs& c, double (&tot)[NV]) {
   __shared__ double sh[NT / 32][NV];
-  __shared__ double sh2[NT][NV];
+  __shared__ double sh2[NV];
   __shared__ bool am_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
@@ -749,17 +758,20 @@ __device__ bool cn_reduce_last(double (&v)[NV], const CnArgs& c, double (&tot)[N
     for (int k = 0; k < NV; ++k) v[k] += ((volatile double*)c.part)[(int64_t)b * CN_NPART + k];
   }
 #pragma unroll
-  for (int k = 0; k < NV; ++k) sh2[threadIdx.x][k] = v[k];
-  __syncthreads();
-  for (int s = NT / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) {
+  for (int k = 0; k < NV; ++k) {
 #pragma unroll
-      for (int k = 0; k < NV; ++k) sh2[threadIdx.x][k] += sh2[threadIdx.x + s][k];
-    }
-    __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    if (lane == 0) sh[wid][k] = v[k];
   }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double s = sh[0][threadIdx.x];
+    for (int w = 1; w < NT / 32; ++w) s += sh[w][threadIdx.x];
+    sh2[threadIdx.x] = s;
+  }
+  __syncthreads();
 #pragma unroll
-  for (int k = 0; k < NV; ++k) tot[k] = sh2[0][k];
+  for (int k = 0; k < NV; ++k) tot[k] = sh2[k];
   if (threadIdx.x == 0) *c.ticket = 0u;
   return true;
 }
@@ -815,35 +827,49 @@ struct DiffStage {
 // explicit step).
 constexpr int OP_STEP = 0, OP_CN_START = 1, OP_CN_APPLY = 2;
 
-// Last-block scalars of a CN stencil pass (mode OP_CN_START or OP_CN_APPLY)
-// from the grid totals: the start of a solve records ||rhs||^2, ||r||^2 and
-// <r, z>_w and tests the warm start; an application forms alpha.
-__device__ __forceinline__ void cn_pass_scalars(const CnArgs& c, int op, const double (&tot)[3]) {
-  if (op == OP_CN_START) {
-    c.scal[CN_BB] = tot[0];
-    c.scal[CN_RR] = tot[1];
-    c.scal[CN_RZ] = tot[2];
-    c.iscal[CI_ITER] = 0;
-    c.iscal[CI_SOLVES] += 1;
-    // converged at the warm start (also a zero right-hand side)
-    c.iscal[CI_DONE] = (tot[1] <= c.tol2 * tot[0] || tot[0] == 0.0) ? 1 : 0;
-  } else {
-    const double pq = tot[0];
-    if (!(pq > 0.0) || !isfinite(pq)) {  // breakdown: keep the current x
-      c.iscal[CI_BREAK] += 1;
-      c.iscal[CI_DONE] = 1;
-    } else {
-      c.scal[CN_PQ] = pq;
-      c.scal[CN_ALPHA] = c.scal[CN_RZ] / pq;
-    }
+// Last-block scalars of a CN stencil pass from the grid totals: the start of
+// a solve records ||rhs||^2 and tests the warm start; an application forms
+// alpha, beta and the stopping decision.
+__device__ __forceinline__ void cn_start_scalars(const CnArgs& c, const double (&tot)[2]) {
+  c.scal[CN_BB] = tot[0];
+  c.scal[CN_RR] = tot[1];
+  c.scal[CN_PEND] = 0.0;
+  c.iscal[CI_ITER] = 0;
+  c.iscal[CI_LOOP] = 0;
+  c.iscal[CI_SOLVES] += 1;
+  // converged at the warm start (also a zero right-hand side)
+  c.iscal[CI_DONE] = (tot[1] <= c.tol2 * tot[0] || tot[0] == 0.0) ? 1 : 0;
+}
+__device__ __forceinline__ void cn_apply_scalars(const CnArgs& c, const double (&tot)[7]) {
+  const double pq = tot[0], rz = tot[4];
+  if (!(pq > 0.0) || !isfinite(pq)) {  // breakdown: keep the current x
+    c.iscal[CI_BREAK] += 1;
+    c.iscal[CI_DONE] = 1;
+    return;
+  }
+  const float alpha = (float)(rz / pq);
+  const double al = alpha;
+  const double rz_new = rz + al * (al * tot[6] - 2.0 * tot[5]);
+  const double rr = tot[1] + al * (al * tot[3] - 2.0 * tot[2]);
+  const int it = c.iscal[CI_ITER] + 1;
+  c.iscal[CI_ITER] = it;
+  c.iscal[CI_TOTAL] += 1;
+  c.scal[CN_ALPHA] = al;
+  c.scal[CN_BETA] = rz > 0.0 ? rz_new / rz : 0.0;
+  c.scal[CN_RR] = rr;
+  const bool below = rr <= c.tol2 * c.scal[CN_BB];
+  if (below || it >= c.max_iter || !isfinite(rr)) {
+    if (!below) c.iscal[CI_UNCONV] += 1;
+    c.scal[CN_PEND] = al;
+    c.iscal[CI_DONE] = 1;
   }
 }
 
 // Persistent diffusion pass over bricks (then chunks of BV Purkinje nodes),
 // tiles double-buffered with cp.async.  OP_STEP: the explicit diffusion half
 // of the split step (V_{i+1} from W_i, outputs of step i).  OP_CN_START: the
-// start of a theta-scheme solve on W_i (x = W, r = Lh W, p = Dinv r and
-// their sums).  OP_CN_APPLY: q = p - theta Lh p and <p, q>_w.  The CN
+// start of a theta-scheme solve on W_i (x = W, r = Lh W, p = Dinv r, ||rhs||^2
+// and ||r||^2).  OP_CN_APPLY: q = p - theta Lh p and its seven sums.  The CN
 // passes write tissue entries only: padding entries of the CG vectors are
 // zero from set-up and stay zero.
 template <int BI, int BJ, int BK, bool ANISO, int OP>
@@ -926,7 +952,24 @@ __device__ __forceinline__ void diffuse_pass(const MonoArgs a, const CnArgs cn, 
     s_vm_frame = (a.vm_every > 0 && step % a.vm_every == 0) ? step / a.vm_every : -1;
     s_anim_frame = (a.frame_every > 0 && step % a.frame_every == 0) ? step / a.frame_every : -1;
   }
-  double v[3] = {0.0, 0.0, 0.0};  // CN sums
+  constexpr int NV = OP == OP_CN_APPLY ? 7 : 2;
+  double v[NV];  // CN sums
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  // the seven sums of an application at one entry
+  auto sums = [&](float pi, float qi, float ri, float di, float w) {
+    if constexpr (OP == OP_CN_APPLY) {
+      const double wd = (double)w * di, rr = (double)ri * ri, rq = (double)ri * qi,
+                   qq = (double)qi * qi;
+      v[0] += (double)w * pi * qi;
+      v[1] += rr;
+      v[2] += rq;
+      v[3] += qq;
+      v[4] += wd * rr;
+      v[5] += wd * rq;
+      v[6] += wd * qq;
+    }
+  };
   // item m of this CTA is blockIdx.x + m G_, staged in stage m % NS; its
   // neighbour list sits in ring slot m % RS, fetched together with item
   // m - (NS - 1) (the first NS - 1 lists are loaded directly), so it is
@@ -972,6 +1015,11 @@ __device__ __forceinline__ void diffuse_pass(const MonoArgs a, const CnArgs cn, 
           const float Vn = diffuse<G::SI, G::SJ, G::NT, ANISO>(a, st, tW, tD, c, tag, slot, odd);
           voxel_outputs(a, slot, tag, Vn, st[D::VP + tid], step, s_vm_frame, s_anim_frame);
         } else {
+          float ri = 0.0f, di = 0.0f;
+          if constexpr (OP == OP_CN_APPLY) {  // in flight during the stencil
+            ri = cn.r[slot];
+            di = cn.dinv[slot];
+          }
           const float acc = stencil_acc<G::SI, G::SJ, G::NT, ANISO>(a, st, tW, tD, c, tag, slot, Wpk);
           if constexpr (OP == OP_CN_START) {
             const float Wi = st[c], z = st[D::VP + tid] * acc, b = Wi + cn.omt * acc;
@@ -980,11 +1028,10 @@ __device__ __forceinline__ void diffuse_pass(const MonoArgs a, const CnArgs cn, 
             cn.p[slot] = z;
             v[0] += (double)b * b;
             v[1] += (double)acc * acc;
-            v[2] += (double)acc * z;
           } else {
             const float pi = st[c], qi = pi - cn.theta * acc;
             cn.q[slot] = qi;
-            v[0] += (double)pi * qi;
+            sums(pi, qi, ri, di, 1.0f);
           }
         }
       }
@@ -996,7 +1043,6 @@ __device__ __forceinline__ void diffuse_pass(const MonoArgs a, const CnArgs cn, 
         } else {
           const float acc = purkinje_acc(a, p, Wpk, Win);
           const int64_t e = a.n_slots + p;
-          const float w = cn.pk_weight;
           if constexpr (OP == OP_CN_START) {
             const float Wi = Wpk[p], z = cn.dinv[e] * acc, b = Wi + cn.omt * acc;
             cn.x[e] = Wi;
@@ -1004,11 +1050,10 @@ __device__ __forceinline__ void diffuse_pass(const MonoArgs a, const CnArgs cn, 
             cn.p[e] = z;
             v[0] += (double)b * b;
             v[1] += (double)acc * acc;
-            v[2] += (double)w * acc * z;
           } else {
             const float pi = Wpk[p], qi = pi - cn.theta * acc;
             cn.q[e] = qi;
-            v[0] += (double)w * pi * qi;
+            sums(pi, qi, cn.r[e], cn.dinv[e], cn.pk_weight);
           }
         }
       }
@@ -1017,8 +1062,11 @@ __device__ __forceinline__ void diffuse_pass(const MonoArgs a, const CnArgs cn, 
   }
   cp_async_wait_all();
   if constexpr (OP != OP_STEP) {
-    double tot[3];
-    if (cn_reduce_last<BV, 3>(v, cn, tot) && threadIdx.x == 0) cn_pass_scalars(cn, OP, tot);
+    double tot[NV];
+    if (cn_reduce_last<BV, NV>(v, cn, tot) && threadIdx.x == 0) {
+      if constexpr (OP == OP_CN_START) cn_start_scalars(cn, tot);
+      else cn_apply_scalars(cn, tot);
+    }
   }
 }
 
@@ -1057,6 +1105,7 @@ __global__ void __launch_bounds__(ION_THREADS, 8) mono_ionic_kernel(MonoArgs a, 
     }
     __syncthreads();
   }
+  const float pend = mode == 2 ? (float)*a.cn_pend : 0.0f;  // the solve's last step
   const bool odd = step & 1;
   const int64_t istep = mode == 1 ? 0 : step + 1;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1065,7 +1114,7 @@ __global__ void __launch_bounds__(ION_THREADS, 8) mono_ionic_kernel(MonoArgs a, 
     const uint32_t tag = a.tag[slot];
     float Vn;
     if constexpr (mode == 2) {
-      Vn = fminf(fmaxf(a.cn_x[slot], -150.0f), 80.0f);
+      Vn = fminf(fmaxf(a.cn_x[slot] + pend * a.cn_p[slot], -150.0f), 80.0f);
       voxel_outputs(a, slot, tag, Vn, a.Vpost[slot], step, s_vm_frame, s_anim_frame);
     } else {
       Vn = a.Vpost[slot];
@@ -1087,7 +1136,7 @@ __global__ void __launch_bounds__(ION_THREADS, 8) mono_ionic_kernel(MonoArgs a, 
     if (p >= 0 && p < a.n_pk) {
       float Vn;
       if constexpr (mode == 2) {
-        Vn = fminf(fmaxf(a.cn_x[a.n_slots + p], -150.0f), 80.0f);
+        Vn = fminf(fmaxf(a.cn_x[a.n_slots + p] + pend * a.cn_p[a.n_slots + p], -150.0f), 80.0f);
         a.pk_Vpost[p] = Vn;
         if (s_anim_frame >= 0) a.pk_frames[s_anim_frame * (int64_t)a.n_pk + p] = Vn;
       } else {
@@ -1143,60 +1192,26 @@ __global__ void __launch_bounds__(BI * BJ * BK) cn_diag_kernel(MonoArgs a, CnArg
   }
 }
 
-// x += alpha p, r -= alpha q; sums ||r||^2 and <r, Dinv r>_w; the last block
-// takes beta and the stopping decision.
-__global__ void __launch_bounds__(CN_TB) cn_update_kernel(CnArgs c, int64_t ns) {
-  if (c.iscal[CI_DONE]) return;
-  const float alpha = (float)c.scal[CN_ALPHA];
-  double v[2] = {0.0, 0.0};
+// x += alpha p, r -= alpha q, p = Dinv r + beta p.  In a solve captured in a
+// CUDA graph this ends the body of the conditional WHILE node `loop` (0: none)
+// and sets whether it runs again: not converged, and fewer than max_iter
+// iterations by its own counter, which bounds the loop whatever the other
+// kernels do.
+__global__ void __launch_bounds__(CN_TB) cn_update_kernel(CnArgs c, cudaGraphConditionalHandle loop) {
+  const bool done = c.iscal[CI_DONE];
+  if (loop && blockIdx.x == 0 && threadIdx.x == 0) {
+    const int n = ++c.iscal[CI_LOOP];
+    cudaGraphSetConditional(loop, (!done && n < c.max_iter) ? 1u : 0u);
+  }
+  if (done) return;
+  const float alpha = (float)c.scal[CN_ALPHA], beta = (float)c.scal[CN_BETA];
   for (int64_t e = blockIdx.x * (int64_t)CN_TB + threadIdx.x; e < c.n;
        e += (int64_t)gridDim.x * CN_TB) {
-    const float xi = c.x[e] + alpha * c.p[e];
-    const float ri = c.r[e] - alpha * c.q[e];
-    c.x[e] = xi;
+    const float pi = c.p[e], ri = c.r[e] - alpha * c.q[e];
+    c.x[e] = c.x[e] + alpha * pi;
     c.r[e] = ri;
-    const float z = c.dinv[e] * ri;
-    v[0] += (double)ri * ri;
-    v[1] += (double)(e < ns ? 1.0f : c.pk_weight) * ri * z;
+    c.p[e] = __fmaf_rn(beta, pi, __fmul_rn(c.dinv[e], ri));
   }
-  double tot[2];
-  if (!cn_reduce_last<CN_TB, 2>(v, c, tot)) return;
-  if (threadIdx.x != 0) return;
-  const int it = c.iscal[CI_ITER] + 1;
-  c.iscal[CI_ITER] = it;
-  c.iscal[CI_TOTAL] += 1;
-  c.scal[CN_RR] = tot[0];
-  const double rz_old = c.scal[CN_RZ];
-  c.scal[CN_BETA] = rz_old > 0.0 ? tot[1] / rz_old : 0.0;
-  c.scal[CN_RZ] = tot[1];
-  if (tot[0] <= c.tol2 * c.scal[CN_BB]) {
-    c.iscal[CI_DONE] = 1;
-  } else if (it >= c.max_iter || !isfinite(tot[0])) {
-    c.iscal[CI_UNCONV] += 1;
-    c.iscal[CI_DONE] = 1;
-  }
-}
-
-// p = Dinv r + beta p.
-__global__ void __launch_bounds__(CN_TB) cn_dir_kernel(CnArgs c) {
-  if (c.iscal[CI_DONE]) return;
-  const float beta = (float)c.scal[CN_BETA];
-  for (int64_t e = blockIdx.x * (int64_t)CN_TB + threadIdx.x; e < c.n;
-       e += (int64_t)gridDim.x * CN_TB)
-    c.p[e] = c.dinv[e] * c.r[e] + beta * c.p[e];
-}
-
-// Loop condition of a solve captured in a CUDA graph (a conditional WHILE
-// node): before the loop (init) "not yet converged", after each iteration
-// "not converged and fewer than max_iter iterations".  Its own counter
-// bounds the loop whatever the other kernels do.
-__global__ void cn_cond_kernel(cudaGraphConditionalHandle hd, CnArgs c, int init) {
-  int n = 0;
-  if (init)
-    c.iscal[CI_LOOP] = 0;
-  else
-    n = ++c.iscal[CI_LOOP];
-  cudaGraphSetConditional(hd, (!c.iscal[CI_DONE] && n < c.max_iter) ? 1u : 0u);
 }
 
 }  // namespace hp
@@ -1536,19 +1551,20 @@ static hp_status setup_cn(HpMono* h, const ShapeEntry* se, const HpMonoDesc* d, 
   // padding entries of the CG vectors stay zero (the passes skip them)
   for (float* v : {c.x, c.r, c.p, c.q}) HP_CUDA_TRY(cudaMemsetAsync(v, 0, n * sizeof(float), s));
   h->a.cn_x = c.x;
+  h->a.cn_p = c.p;
+  h->a.cn_pend = c.scal + CN_PEND;
   h->cn<<<h->cn_grid, h->bv, 0, s>>>(h->a, c);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
 
-// One CG iteration of the theta-scheme solve: q = M p (tiled pass, alpha),
-// x and r updates (beta, stopping test), new direction.  Every kernel
-// returns at once once the done flag is set.
-static void cn_iteration(HpMono* h, cudaStream_t s) {
+// One CG iteration of the theta-scheme solve: q = M p (tiled pass: alpha, beta,
+// stopping test), then x, r and p.  Both return at once once the done flag is
+// set.
+static void cn_iteration(HpMono* h, cudaGraphConditionalHandle loop, cudaStream_t s) {
   const CnArgs& c = h->cn_a;
   h->cn_apply<<<h->cn_pgrid, h->bv, h->diff_smem, s>>>(h->a, c);
-  cn_update_kernel<<<h->cn_vgrid, CN_TB, 0, s>>>(c, h->a.n_slots);
-  cn_dir_kernel<<<h->cn_vgrid, CN_TB, 0, s>>>(c);
+  cn_update_kernel<<<h->cn_vgrid, CN_TB, 0, s>>>(c, loop);
 }
 
 // One theta-scheme step: the stencil pass that starts the solve, CG
@@ -1562,7 +1578,7 @@ static hp_status cn_step(HpMono* h, cudaStream_t s) {
   int launched = 0;
   while (launched < c.max_iter) {
     const int k = std::min(h->cn_chunk, c.max_iter - launched);
-    for (int j = 0; j < k; ++j) cn_iteration(h, s);
+    for (int j = 0; j < k; ++j) cn_iteration(h, 0, s);
     HP_CUDA_TRY(cudaGetLastError());
     launched += k;
     HP_CUDA_TRY(cudaMemcpyAsync(h->cn_host, c.iscal + CI_DONE, 2 * sizeof(int32_t),
@@ -1579,10 +1595,10 @@ static hp_status cn_step(HpMono* h, cudaStream_t s) {
 }
 
 // Captures n theta-scheme steps on s (which is capturing): per step the
-// start pass, the loop-condition kernel and a conditional WHILE node whose
-// body (captured on cn_body_stream) is one CG iteration plus the condition
-// update, then the outputs, the ionic half and the step count.  No host
-// round trip per step.
+// start pass and a conditional WHILE node whose body (captured on
+// cn_body_stream) is one CG iteration, entered at least once (its kernels
+// return at once where the warm start converged), then the outputs, the ionic
+// half and the step count.  No host round trip per step.
 static hp_status cn_capture_steps(HpMono* h, int n, cudaStream_t s) {
   const CnArgs& c = h->cn_a;
   cudaStream_t sb = h->cn_body_stream;
@@ -1594,9 +1610,7 @@ static hp_status cn_capture_steps(HpMono* h, int n, cudaStream_t s) {
     size_t nd = 0;
     HP_CUDA_TRY(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
     cudaGraphConditionalHandle hd;
-    HP_CUDA_TRY(cudaGraphConditionalHandleCreate(&hd, g, 0, 0));
-    cn_cond_kernel<<<1, 1, 0, s>>>(hd, c, 1);
-    HP_CUDA_TRY(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
+    HP_CUDA_TRY(cudaGraphConditionalHandleCreate(&hd, g, 1, cudaGraphCondAssignDefault));
     cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
     np.conditional.handle = hd;
     np.conditional.type = cudaGraphCondTypeWhile;
@@ -1606,8 +1620,7 @@ static hp_status cn_capture_steps(HpMono* h, int n, cudaStream_t s) {
     cudaGraph_t body = np.conditional.phGraph_out[0];
     HP_CUDA_TRY(cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0,
                                               cudaStreamCaptureModeRelaxed));
-    cn_iteration(h, sb);
-    cn_cond_kernel<<<1, 1, 0, sb>>>(hd, c, 0);
+    cn_iteration(h, hd, sb);
     cudaGraph_t bo = nullptr;
     HP_CUDA_TRY(cudaStreamEndCapture(sb, &bo));
     HP_CUDA_TRY(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));

@@ -11,18 +11,43 @@
 namespace hp {
 namespace tc {
 
+// One input line (130 voxels: a tile and its halo) in shared memory as the
+// forward kernels' K-major A operand: a row of 32, 64 or 128 bytes a voxel in
+// the swizzle of that width; 48 and 96 channels are three sub-lines of 32 and
+// 64 bytes a voxel.  A TMA box of 8 channels, the unswizzled core matrices,
+// fetches the same line as CIN / 8 rows of 16 bytes a voxel: 48 -> 16 at
+// 64 x 56 x 128 64 us against 58, 96 -> 32 at 32 x 28 x 128 56.5 against 55.5.
+// The swizzle permutes 16-byte columns by address bits, so moving the
+// descriptor's start by a voxel row (dx) or by 32 bytes (the next 16 channels)
+// needs no other change.
+template <int CIN>
+struct ALine {
+  static constexpr int RB = CIN % 64 == 0 ? 128 : (CIN % 32 == 0 ? 64 : 32);  // bytes a row
+  static constexpr int CH = RB / 2;                     // channels a sub-line
+  static constexpr int SUB = CIN / CH;                  // sub-lines
+  static constexpr int ALIGN = 8 * RB;                  // the swizzle pattern's period
+  static constexpr int SUB_BYTES = (LINE + 7) / 8 * ALIGN;
+  static constexpr int BYTES = SUB * SUB_BYTES;
+  static constexpr int TX = SUB * LINE * RB;
+  // byte offset of 16-channel group k
+  __host__ __device__ static constexpr int k_off(int k) {
+    return 32 * k / RB * SUB_BYTES + 32 * k % RB;
+  }
+};
+
 template <int CIN, int COUT>
 struct ConvCfg {
+  using A = ALine<CIN>;
   static constexpr int G = CIN / 8;
-  static constexpr int A_BYTES = G * CHUNK;
-  static constexpr int A_TX = G * LINE * 16;
+  static constexpr int A_BYTES = A::BYTES;
+  static constexpr int A_TX = A::TX;
   static constexpr int B_BYTES = 3 * CIN * COUT * 2;
   static constexpr int STAGE = A_BYTES + B_BYTES;
-  static constexpr int SMEM = 2 * STAGE + 128;
+  static constexpr int SMEM = 2 * STAGE + A::ALIGN;
   static constexpr uint32_t COLS = TmemCols<COUT>::value;
   static constexpr uint32_t IDESC = idesc_bf16(TILE_M, COUT);
   static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 256, "channel counts");
-  static_assert(B_BYTES % 128 == 0, "stage alignment");
+  static_assert(STAGE % A::ALIGN == 0, "stage alignment");
 };
 
 template <int CIN, int COUT>
@@ -32,13 +57,14 @@ conv3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat16* __
                 const __nv_bfloat16* __restrict__ mask, int D, int H, int W, int epi, int* err) {
   using C = ConvCfg<CIN, COUT>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
+  uint8_t* smem =
+      (uint8_t*)(((uintptr_t)smem_raw + C::A::ALIGN - 1) & ~(uintptr_t)(C::A::ALIGN - 1));
   __shared__ __align__(8) uint64_t full[2];
   __shared__ __align__(8) uint64_t empty[2];
   __shared__ __align__(8) uint64_t done;
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int w0 = blockIdx.x * TILE_M, h = blockIdx.y, d = blockIdx.z;
 
   if (tid == 0) {
@@ -54,63 +80,72 @@ conv3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat16* __
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
 
-  if (tid == 0) {
+  if (warp == 0) {
+    // the warp stays converged; one elected lane issues copies and products
     auto issue = [&](int s, int buf) {
       const int dz = s / 3 - 1, dy = s % 3 - 1;
       uint8_t* A = smem + buf * C::STAGE;
       uint8_t* B = A + C::A_BYTES;
       mbar_expect_tx(&full[buf], C::A_TX + C::B_BYTES);
 #pragma unroll
-      for (int g = 0; g < C::G; ++g)
-        tma_load_4d(A + g * CHUNK, &tmX, g * 8, w0 - 1, h + dy, d + dz, &full[buf]);
+      for (int g = 0; g < C::A::SUB; ++g)
+        tma_load_4d(A + g * C::A::SUB_BYTES, &tmX, g * C::A::CH, w0 - 1, h + dy, d + dz,
+                    &full[buf]);
       const int tap0 = 9 * (dz + 1) + 3 * (dy + 1);
       bulk_load(B, Wp + (size_t)tap0 * CIN * COUT, C::B_BYTES, &full[buf]);
     };
-    int issued = 0;
-    issue(0, 0);
-    issue(1, 1);
-    issued = 2;
-    int consumed = 0;
+    if (elect_one()) {
+      issue(0, 0);
+      issue(1, 1);
+    }
+    __syncwarp();
+    int issued = 2, consumed = 0, code = 0;
     for (int s = 0; s < 9; ++s) {
       const int buf = s & 1;
       const uint32_t par = (s >> 1) & 1;
-      if (!mbar_wait(&full[buf], par)) {
-        atomicOr(err, 1);
-        failed = 1;
+      if (!mbar_wait_warp(&full[buf], par)) {
+        code = 1;
         break;
       }
       tc_fence_after();
       const uint32_t a0 = smem_u32(smem + buf * C::STAGE);
-      const uint64_t a_d = smem_desc(a0, CHUNK, 128);
+      const uint64_t a_d = smem_desc_sw<C::A::RB>(a0);
       const uint64_t b_d = smem_desc(a0 + C::A_BYTES, COUT * 16, 128);
+      if (elect_one()) {
 #pragma unroll
-      for (int dx = 0; dx < 3; ++dx) {
+        for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-        for (int k = 0; k < CIN / 16; ++k) {
-          const uint64_t ad = desc_add(a_d, 2 * k * CHUNK + dx * 16);
-          const uint64_t bd = desc_add(b_d, (dx * C::G + 2 * k) * COUT * 16);
-          mma_bf16(tmem, ad, bd, C::IDESC, (s | dx | k) != 0);
-        }
+          for (int k = 0; k < CIN / 16; ++k)
+            mma_bf16(tmem, desc_add(a_d, C::A::k_off(k) + dx * C::A::RB),
+                     desc_add(b_d, (dx * C::G + 2 * k) * COUT * 16), C::IDESC,
+                     (s | dx | k) != 0);
+        mma_commit(&empty[buf]);
       }
-      mma_commit(&empty[buf]);
+      __syncwarp();
       consumed = s + 1;
       if (s + 2 < 9) {
-        if (!mbar_wait(&empty[buf], par)) {
-          atomicOr(err, 2);
-          failed = 1;
+        if (!mbar_wait_warp(&empty[buf], par)) {
+          code = 2;
           break;
         }
-        issue(s + 2, buf);
+        if (elect_one()) issue(s + 2, buf);
+        __syncwarp();
         ++issued;
       }
     }
-    if (failed) {
+    if (code) {
       // let the copies already issued land before the CTA releases smem
-      for (int s = consumed; s < issued; ++s) (void)mbar_wait(&full[s & 1], (s >> 1) & 1);
+      for (int s = consumed; s < issued; ++s) (void)mbar_wait_warp(&full[s & 1], (s >> 1) & 1);
     }
-    mma_commit(&done);
+    if (elect_one()) {
+      if (code) {
+        atomicOr(err, code);
+        failed = 1;
+      }
+      mma_commit(&done);
+    }
   }
   __syncthreads();
   const bool ok = mbar_wait(&done, 0) && !failed;
@@ -158,15 +193,68 @@ conv3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat16* __
   if (warp == 0) tmem_dealloc(tmem, C::COLS);
 }
 
+// The products of input line ri (h0 - 1 + ri) of a depth slice.  It feeds the
+// output lines r within one row of it, by tap row dy = ri - 1 - r.  The tap
+// rows are neighbours in the weight block ([dx][CIN/8][dy][COUT][8]) and
+// output line r accumulates in columns (R - 1 - r) COUT.., so one product with
+// N = 3 COUT does all three (as many as fit N = 256).  A product of 128 rows
+// by 16 channels takes about 50 clocks of an SM at N = 16 and hardly more at
+// 48 -- reading A, not the arithmetic --, so a narrow layer wants few and wide
+// ones: 16 -> 16 at 64 x 56 x 128 20.6 us against 25.1 with a product for each
+// tap row, 48 -> 16 39.3 against 57.5, 96 -> 32 at 32 x 28 x 128 34.9 against
+// 39.6.
+// Within each output line the order of the taps is (dz, dy, dx, channels).
+// `first` marks the first depth slice, whose first product into a line (dy -1,
+// dx 0, channel group 0) overwrites the accumulator.
+template <int CIN, int COUT, int R>
+__device__ __forceinline__ void issue_line(uint32_t acc0, uint64_t a_d, uint64_t b_d, int ri,
+                                           bool first) {
+  using A = ALine<CIN>;
+  constexpr int NT = 256 / COUT < 3 ? 256 / COUT : 3;   // tap rows a product
+  const int r_hi = ri < R ? ri : R - 1, r_lo = ri > 2 ? ri - 2 : 0;
+  const int dy_lo = ri - 1 - r_hi, n_dy = r_hi - r_lo + 1;
+#pragma unroll
+  for (int q0 = 0; q0 < 3; q0 += NT) {
+    if (q0 >= n_dy) continue;
+    const int n = n_dy - q0 < NT ? n_dy - q0 : NT;
+    const uint32_t td = acc0 + (uint32_t)((R - 1 - r_hi + q0) * COUT);
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int k = 0; k < CIN / 16; ++k) {
+        const uint64_t ad = desc_add(a_d, A::k_off(k) + dx * A::RB);
+        const uint64_t bd =
+            desc_add(b_d, ((dx * (CIN / 8) + 2 * k) * 3 + dy_lo + 1 + q0) * COUT * 16);
+        if (first && dy_lo + q0 == -1 && dx == 0 && k == 0) {
+          mma_bf16(td, ad, bd, idesc_bf16(TILE_M, COUT), 0u);
+          if (n > 1)
+            mma_bf16(td + COUT, ad, desc_add(bd, COUT * 16), idesc_bf16(TILE_M, (n - 1) * COUT),
+                     1u);
+        } else {
+          mma_bf16(td, ad, bd, idesc_bf16(TILE_M, n * COUT), 1u);
+        }
+      }
+  }
+}
+
+// The nine taps of depth slice zi to dst as [dx][CIN/8][dy][COUT][8].
+template <int CIN, int COUT>
+__device__ __forceinline__ void load_taps(uint8_t* dst, const CUtensorMap* tmB, int zi,
+                                          uint64_t* bar) {
+#pragma unroll
+  for (int q = 0; q < 3 * (CIN / 8); ++q)
+    tma_load_5d(dst + q * 3 * COUT * 16, tmB, 0, 0, q % (CIN / 8), 9 * zi + q / (CIN / 8), 0, bar);
+}
+
 // -------------------------------------------------------------------------
 // Row-blocked variant: one CTA computes R output lines (h0 .. h0+R-1 at the
 // same (d, w0..w0+127)), one TMEM accumulator of COUT FP32 columns per line.
-// One thread issues the copies up to NS stages ahead, another the products
-// (copy latency no longer serialises with the products' completion).
+// One thread issues the copies up to NS stages ahead, one lane of warp 0 the
+// products (copy latency does not serialise with the products' completion).
 // The K loop runs over dz and the R+2 input lines h0-1 .. h0+R of that
 // depth slice: each input line is loaded once and feeds every output line
 // within one row of it (up to three), and the 9 (dy, dx) taps of a depth
-// slice arrive in one bulk copy per slice -- against one line tile per CTA,
+// slice arrive once per slice -- against one line tile per CTA,
 // which loads every input line three times per depth slice and the weights
 // nine times.  Two weight buffers (slice zi uses buffer zi & 1; a buffer is
 // rewritten only after the MMAs of every stage that read it have completed,
@@ -174,42 +262,44 @@ conv3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat16* __
 // complete in order).
 template <int CIN, int COUT, int R>
 struct RowsCfg {
+  using A = ALine<CIN>;
   static constexpr int G = CIN / 8;
-  static constexpr int A_BYTES = G * CHUNK;
-  static constexpr int A_TX = G * LINE * 16;
+  static constexpr int A_BYTES = A::BYTES;
+  static constexpr int A_TX = A::TX;
   static constexpr int B_BYTES = 9 * CIN * COUT * 2;
-  static constexpr int ACC = (COUT + 31) / 32 * 32;   // TMEM columns per output line
+  static constexpr int ACC = COUT;                    // TMEM columns per output line
   static constexpr uint32_t COLS = R * ACC <= 32 ? 32 : (R * ACC <= 64 ? 64 : (R * ACC <= 128 ? 128 : (R * ACC <= 256 ? 256 : 512)));
   // line stages in flight: four where that keeps the CTA's shared memory
   // small (48 KB), else two (more CTAs per SM measured faster there)
-  static constexpr int NS = 4 * A_BYTES + 2 * B_BYTES + 128 <= 48 * 1024 ? 4 : 2;
-  static constexpr int SMEM = NS * A_BYTES + 2 * B_BYTES + 128;
+  static constexpr int NS = 4 * A_BYTES + 2 * B_BYTES + A::ALIGN <= 48 * 1024 ? 4 : 2;
+  static constexpr int SMEM = NS * A_BYTES + 2 * B_BYTES + A::ALIGN;
   static constexpr int NSTG = 3 * (R + 2);
-  static constexpr uint32_t IDESC = idesc_bf16(TILE_M, COUT);
   static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 256, "channel counts");
   static_assert(R * ACC <= 512, "TMEM columns");
-  static_assert(B_BYTES % 128 == 0 && A_BYTES % 128 == 0, "stage alignment");
+  static_assert(B_BYTES % 128 == 0 && A_BYTES % A::ALIGN == 0, "stage alignment");
 };
 
 constexpr int CONV_ROWS = 4;
 
 template <int CIN, int COUT, int R>
 __global__ void __launch_bounds__(128)
-conv3_tc_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat16* __restrict__ Wp,
-                     const float* __restrict__ bias, void* __restrict__ Yv,
+conv3_tc_rows_kernel(const __grid_constant__ CUtensorMap tmX,
+                     const __grid_constant__ CUtensorMap tmB, const float* __restrict__ bias,
+                     void* __restrict__ Yv,
                      const __nv_bfloat16* __restrict__ mask, int D, int H, int W, int epi,
                      int* err) {
   using C = RowsCfg<CIN, COUT, R>;
   constexpr int NS = C::NS;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
+  uint8_t* smem =
+      (uint8_t*)(((uintptr_t)smem_raw + C::A::ALIGN - 1) & ~(uintptr_t)(C::A::ALIGN - 1));
   __shared__ __align__(8) uint64_t full[NS];
   __shared__ __align__(8) uint64_t empty[NS];
   __shared__ __align__(8) uint64_t done;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int failed;
   __shared__ int issued_s, consumed_s;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int w0 = blockIdx.x * TILE_M, h0 = blockIdx.y * R, d = blockIdx.z;
 
   if (tid == 0) {
@@ -227,7 +317,7 @@ conv3_tc_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat1
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
   uint8_t* const Bbase = smem + NS * C::A_BYTES;
 
   // Producer (thread 32): line stage s goes to buffer s % NS; it is
@@ -250,50 +340,46 @@ conv3_tc_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat1
       const bool new_slice = ri == 0;
       mbar_expect_tx(&full[buf], C::A_TX + (new_slice ? C::B_BYTES : 0));
 #pragma unroll
-      for (int g = 0; g < C::G; ++g)
-        tma_load_4d(A + g * CHUNK, &tmX, g * 8, w0 - 1, h0 - 1 + ri, d + zi - 1, &full[buf]);
+      for (int g = 0; g < C::A::SUB; ++g)
+        tma_load_4d(A + g * C::A::SUB_BYTES, &tmX, g * C::A::CH, w0 - 1, h0 - 1 + ri, d + zi - 1,
+                    &full[buf]);
       if (new_slice)
-        bulk_load(Bbase + (zi & 1) * C::B_BYTES, Wp + (size_t)9 * zi * CIN * COUT, C::B_BYTES,
-                  &full[buf]);
+        load_taps<CIN, COUT>(Bbase + (zi & 1) * C::B_BYTES, &tmB, zi, &full[buf]);
     }
     issued_s = s;
   }
-  // MMA issuer (thread 0)
-  if (tid == 0) {
+  // MMA issuer (warp 0, one elected lane).  The line index is unrolled, so a
+  // product's operands are a base and a constant.
+  if (warp == 0) {
     int s = 0;
-    for (; s < C::NSTG; ++s) {
-      const int buf = s % NS;
-      if (failed || !mbar_wait(&full[buf], (s / NS) & 1)) {
+    bool ok = true;
+    for (int zi = 0; zi < 3 && ok; ++zi) {
+      const uint64_t b_d = smem_desc(smem_u32(Bbase + (zi & 1) * C::B_BYTES), 3 * COUT * 16, 128);
+#pragma unroll
+      for (int ri = 0; ri < R + 2; ++ri) {
+        const int buf = s % NS;
+        if (!mbar_wait_warp(&full[buf], (s / NS) & 1)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint64_t a_d = smem_desc_sw<C::A::RB>(smem_u32(smem + buf * C::A_BYTES));
+        if (elect_one()) {
+          issue_line<CIN, COUT, R>(tmem, a_d, b_d, ri, zi == 0);
+          mma_commit(&empty[buf]);
+        }
+        __syncwarp();
+        ++s;
+      }
+    }
+    if (elect_one()) {
+      if (!ok) {
         atomicOr(err, 1);
         failed = 1;
-        break;
       }
-      tc_fence_after();
-      const int zi = s / (R + 2), ri = s % (R + 2);
-      const uint64_t a_d = smem_desc(smem_u32(smem + buf * C::A_BYTES), CHUNK, 128);
-      const uint64_t b_d = smem_desc(smem_u32(Bbase + (zi & 1) * C::B_BYTES), COUT * 16, 128);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int dy = ri - 1 - r;   // input line h0-1+ri feeds output line h0+r
-        if (dy < -1 || dy > 1) continue;
-        const uint32_t td = tmem + (uint32_t)(r * C::ACC);
-#pragma unroll
-        for (int dx = 0; dx < 3; ++dx) {
-#pragma unroll
-          for (int k = 0; k < CIN / 16; ++k) {
-            const uint64_t ad = desc_add(a_d, 2 * k * CHUNK + dx * 16);
-            const uint64_t bd =
-                desc_add(b_d, ((3 * (dy + 1) + dx) * C::G + 2 * k) * COUT * 16);
-            // the first product into line r (zi 0, dy -1, dx 0, k 0) overwrites
-            const uint32_t acc = (zi != 0 || dy != -1 || dx != 0 || k != 0) ? 1u : 0u;
-            mma_bf16(td, ad, bd, C::IDESC, acc);
-          }
-        }
-      }
-      mma_commit(&empty[buf]);
+      consumed_s = s;
+      mma_commit(&done);
     }
-    consumed_s = s;
-    mma_commit(&done);
   }
   __syncthreads();
   if (tid == 32 && failed) {
@@ -310,7 +396,7 @@ conv3_tc_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat1
 #pragma unroll 1
     for (int r = 0; r < R; ++r) {
       if (h0 + r >= H) break;
-      const uint32_t tl = trow + (uint32_t)(r * C::ACC);
+      const uint32_t tl = trow + (uint32_t)((R - 1 - r) * C::ACC);
       const int64_t vox = ((int64_t)d * H + h0 + r) * W + w0 + tid;
       if (epi == EPI_F32_C0) {
         float v[16];
@@ -376,22 +462,22 @@ conv3_tc_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __nv_bfloat1
 // flight, frees its TMEM and returns.
 template <int CIN, int COUT, int RR>
 struct PersistCfg {
+  using A = ALine<CIN>;
   static constexpr int G = CIN / 8;
-  static constexpr int A_BYTES = G * CHUNK;
-  static constexpr int A_TX = G * LINE * 16;
+  static constexpr int A_BYTES = A::BYTES;
+  static constexpr int A_TX = A::TX;
   static constexpr int B_BYTES = 9 * CIN * COUT * 2;
-  static constexpr int ACC = (COUT + 31) / 32 * 32;          // TMEM columns per output line
+  static constexpr int ACC = COUT;                           // TMEM columns per output line
   static constexpr int R = RR;                                // output lines per tile
   static constexpr int NSTG = 3 * (R + 2);                   // line stages per tile
   static constexpr uint32_t COLS = 2 * R * ACC <= 128 ? 128 : (2 * R * ACC <= 256 ? 256 : 512);
-  static constexpr int NS_FIT = (200 * 1024 - 2 * B_BYTES - 128) / A_BYTES;
+  static constexpr int NS_FIT = (200 * 1024 - 2 * B_BYTES - A::ALIGN) / A_BYTES;
   static constexpr int NS = NS_FIT > R + 2 ? R + 2 : NS_FIT;
-  static constexpr int SMEM = NS * A_BYTES + 2 * B_BYTES + 128;
-  static constexpr uint32_t IDESC = idesc_bf16(TILE_M, COUT);
+  static constexpr int SMEM = NS * A_BYTES + 2 * B_BYTES + A::ALIGN;
   static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 256, "channel counts");
   static_assert(NS >= 2 && NS <= R + 2, "ring depth (the weight-buffer reuse needs NS <= R + 2)");
   static_assert(2 * R * ACC <= 512, "TMEM columns");
-  static_assert(B_BYTES % 128 == 0 && A_BYTES % 128 == 0, "stage alignment");
+  static_assert(B_BYTES % 128 == 0 && A_BYTES % A::ALIGN == 0, "stage alignment");
 };
 
 constexpr int PERSIST_THREADS = 192;
@@ -399,13 +485,14 @@ constexpr int PERSIST_THREADS = 192;
 template <int CIN, int COUT, int RR>
 __global__ void __launch_bounds__(PERSIST_THREADS, 1)
 conv3_tc_persist_kernel(const __grid_constant__ CUtensorMap tmX,
-                        const __nv_bfloat16* __restrict__ Wp, const float* __restrict__ bias,
+                        const __grid_constant__ CUtensorMap tmB, const float* __restrict__ bias,
                         void* __restrict__ Yv, const __nv_bfloat16* __restrict__ mask, int D,
                         int H, int W, int epi, int* err) {
   using C = PersistCfg<CIN, COUT, RR>;
   constexpr int NS = C::NS, R = C::R, NSTG = C::NSTG, ACC = C::ACC;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
+  uint8_t* smem =
+      (uint8_t*)(((uintptr_t)smem_raw + C::A::ALIGN - 1) & ~(uintptr_t)(C::A::ALIGN - 1));
   __shared__ __align__(8) uint64_t full[NS];
   __shared__ __align__(8) uint64_t empty[NS];
   __shared__ __align__(8) uint64_t acc_full[2];
@@ -414,7 +501,7 @@ conv3_tc_persist_kernel(const __grid_constant__ CUtensorMap tmX,
   __shared__ uint32_t tmem_base;
   __shared__ volatile int failed;
   __shared__ int issued_s, consumed_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int n_wt = W / TILE_M, n_hb = (H + R - 1) / R;
   const int n_tiles = n_wt * n_hb * D;
 
@@ -437,7 +524,7 @@ conv3_tc_persist_kernel(const __grid_constant__ CUtensorMap tmX,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
   uint8_t* const Bbase = smem + NS * C::A_BYTES;
   auto fail = [&](int code) {
     atomicOr(err, code);
@@ -463,64 +550,56 @@ conv3_tc_persist_kernel(const __grid_constant__ CUtensorMap tmX,
           const bool new_slice = ri == 0;
           mbar_expect_tx(&full[buf], C::A_TX + (new_slice ? C::B_BYTES : 0));
 #pragma unroll
-          for (int g = 0; g < C::G; ++g)
-            tma_load_4d(A + g * CHUNK, &tmX, g * 8, w0 - 1, h0 - 1 + ri, d + zi - 1, &full[buf]);
+          for (int g = 0; g < C::A::SUB; ++g)
+            tma_load_4d(A + g * C::A::SUB_BYTES, &tmX, g * C::A::CH, w0 - 1, h0 - 1 + ri,
+                        d + zi - 1, &full[buf]);
           if (new_slice)
-            bulk_load(Bbase + ((s / (R + 2)) & 1) * C::B_BYTES, Wp + (size_t)9 * zi * CIN * COUT,
-                      C::B_BYTES, &full[buf]);
+            load_taps<CIN, COUT>(Bbase + ((s / (R + 2)) & 1) * C::B_BYTES, &tmB, zi, &full[buf]);
         }
       }
       issued_s = s;
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // MMA issuer
-      int s = 0, j = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
-        const int b = j & 1;
-        if (j >= 2 && !mbar_wait_f(&acc_empty[b], ((j >> 1) - 1) & 1, &failed)) {
-          fail(8);
-          break;
-        }
-        tc_fence_after();
-        const uint32_t accb = tmem + (uint32_t)(b * R * ACC);
-        for (int st = 0; st < NSTG; ++st, ++s) {
+    // MMA issuer: the warp stays converged, one elected lane issues
+    int s = 0, j = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
+      const int b = j & 1;
+      if (j >= 2 && !__all_sync(0xffffffffu,
+                                mbar_wait_f(&acc_empty[b], ((j >> 1) - 1) & 1, &failed))) {
+        if (lane == 0) fail(8);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t accb = tmem + (uint32_t)(b * R * ACC);
+      for (int zi = 0; zi < 3 && ok; ++zi) {
+        const uint64_t b_d =
+            smem_desc(smem_u32(Bbase + ((s / (R + 2)) & 1) * C::B_BYTES), 3 * COUT * 16, 128);
+#pragma unroll
+        for (int ri = 0; ri < R + 2; ++ri) {
           const int buf = s % NS;
-          if (!mbar_wait_f(&full[buf], (s / NS) & 1, &failed)) {
-            fail(1);
+          if (!__all_sync(0xffffffffu, mbar_wait_f(&full[buf], (s / NS) & 1, &failed))) {
+            if (lane == 0) fail(1);
             ok = false;
             break;
           }
           tc_fence_after();
-          const int zi = st / (R + 2), ri = st % (R + 2);
-          const uint64_t a_d = smem_desc(smem_u32(smem + buf * C::A_BYTES), CHUNK, 128);
-          const uint64_t b_d =
-              smem_desc(smem_u32(Bbase + ((s / (R + 2)) & 1) * C::B_BYTES), COUT * 16, 128);
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int dy = ri - 1 - r;  // input line h0-1+ri feeds output line h0+r
-            if (dy < -1 || dy > 1) continue;
-            const uint32_t td = accb + (uint32_t)(r * ACC);
-#pragma unroll
-            for (int dx = 0; dx < 3; ++dx) {
-#pragma unroll
-              for (int k = 0; k < CIN / 16; ++k) {
-                const uint64_t ad = desc_add(a_d, 2 * k * CHUNK + dx * 16);
-                const uint64_t bd =
-                    desc_add(b_d, ((3 * (dy + 1) + dx) * C::G + 2 * k) * COUT * 16);
-                // the first product into line r (zi 0, dy -1, dx 0, k 0) overwrites
-                const uint32_t acc = (zi != 0 || dy != -1 || dx != 0 || k != 0) ? 1u : 0u;
-                mma_bf16(td, ad, bd, C::IDESC, acc);
-              }
-            }
+          const uint64_t a_d = smem_desc_sw<C::A::RB>(smem_u32(smem + buf * C::A_BYTES));
+          if (elect_one()) {
+            issue_line<CIN, COUT, R>(accb, a_d, b_d, ri, zi == 0);
+            mma_commit(&empty[buf]);
           }
-          mma_commit(&empty[buf]);
+          __syncwarp();
+          ++s;
         }
-        if (!ok) break;
-        mma_commit(&acc_full[b]);
       }
+      if (!ok) break;
+      if (elect_one()) mma_commit(&acc_full[b]);
+      __syncwarp();
+    }
+    // every product issued has completed before the CTA releases TMEM
+    if (elect_one()) {
       consumed_s = s;
-      // every product issued has completed before the CTA releases TMEM
       mma_commit(&done);
       if (!mbar_wait(&done, 0)) atomicOr(err, 4);
     }
@@ -540,7 +619,7 @@ conv3_tc_persist_kernel(const __grid_constant__ CUtensorMap tmX,
 #pragma unroll 1
       for (int r = 0; r < R; ++r) {
         if (h0 + r >= H) break;
-        const uint32_t tl = tlane + (uint32_t)(b * R * ACC + r * ACC);
+        const uint32_t tl = tlane + (uint32_t)((b * R + R - 1 - r) * ACC);
         const int64_t vox = ((int64_t)d * H + h0 + r) * W + w0 + row;
         if (epi == EPI_F32_C0) {
           float v[16];
@@ -610,9 +689,10 @@ static hp_status get_encode() {
   return HP_OK;
 }
 
-// Tensor map over X[D][H][W][C] (bf16) with box (8 ch, box_w voxels, 1, 1).
+// Tensor map over X[D][H][W][C] (bf16) with box (box_c ch, box_w voxels, 1, 1);
+// boxes of 16, 32 and 64 channels land in the swizzle of their row's width.
 hp_status make_line_map(CUtensorMap* map, const void* X, int D, int H, int W, int Cch,
-                        int box_w = LINE) {
+                        int box_w = LINE, int box_c = 8) {
   hp_status s = get_encode();
   if (s != HP_OK) return s;
   if (((uintptr_t)X & 15) != 0) {
@@ -622,9 +702,33 @@ hp_status make_line_map(CUtensorMap* map, const void* X, int D, int H, int W, in
   cuuint64_t dims[4] = {(cuuint64_t)Cch, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D};
   cuuint64_t strides[3] = {(cuuint64_t)Cch * 2, (cuuint64_t)W * Cch * 2,
                            (cuuint64_t)H * W * Cch * 2};
-  cuuint32_t box[4] = {8, (cuuint32_t)box_w, 1, 1};
+  cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)box_w, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUtensorMapSwizzle swizzle = box_c == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                                     : box_c == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                     : box_c == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                                   : CU_TENSOR_MAP_SWIZZLE_NONE;
   CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)X, dims, strides, box,
+                        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    hp::set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return HP_ERR_CUDA;
+  }
+  return HP_OK;
+}
+
+// Tensor map over the packed weights [27][cin/8][cout][8] whose box is the
+// three dy taps of one (dz, dx, channel group) as [dy][cout][8].
+hp_status make_tap_map(CUtensorMap* map, const void* Wp, int cin, int cout) {
+  hp_status s = get_encode();
+  if (s != HP_OK) return s;
+  const cuuint64_t row = (cuuint64_t)cout * 16, tap = row * (cin / 8);
+  cuuint64_t dims[5] = {128, (cuuint64_t)cout / 16, (cuuint64_t)cin / 8, 21, 3};
+  cuuint64_t strides[4] = {256, row, tap, 3 * tap};
+  cuuint32_t box[5] = {128, (cuuint32_t)cout / 16, 1, 1, 3};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void*)Wp, dims, strides, box,
                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -636,33 +740,34 @@ hp_status make_line_map(CUtensorMap* map, const void* X, int D, int H, int W, in
 
 typedef void (*ConvFn)(CUtensorMap, const __nv_bfloat16*, const float*, void*,
                        const __nv_bfloat16*, int, int, int, int, int*);
+typedef void (*ConvLinesFn)(CUtensorMap, CUtensorMap, const float*, void*, const __nv_bfloat16*,
+                            int, int, int, int, int*);
 
 struct ConvEntry {
-  int cin, cout, smem;
+  int cin, cout, box_c, smem;
   ConvFn fn;
   int rows_smem;
-  ConvFn rows_fn;   // CONV_ROWS output lines per CTA
+  ConvLinesFn rows_fn;   // CONV_ROWS output lines per CTA
   int persist_smem;
-  ConvFn persist_fn;   // persistent warp-specialised kernel, or null
+  ConvLinesFn persist_fn;   // persistent warp-specialised kernel, or null
   int persist_rows;
   uint32_t persist_cols;
 };
 
-// Kernel per layer shape, from per-shape timings on B200 (network level
-// sizes, hp_conv3_forward, CUDA events): the persistent kernel with two
-// output lines per tile wins on the wide layers (96 -> 32 95 against
-// 134 us, 32 -> 96 55 against 73, 64 -> 64 29 against 35, 64 -> 32 25
-// against 31) and loses on the narrow ones (16 -> 16 108-118 against 54,
-// 48 -> 16 195 against 125, 32 -> 32 49 against 35): one CTA per SM
-// pair of copy and MMA threads keeps fewer small products in flight than
-// four row-blocked CTAs.
+// Kernel per layer shape, from timings of hp_conv3_forward (cold L2, CUDA
+// events) at 32 x 28 x 128 and 64 x 56 x 128: with few input channels a
+// product chain is short and row-blocked CTAs, several on an SM, hide its
+// waits (16 -> 16 22.6 us against 38.4 for the persistent kernel, 48 -> 16
+// 49.2 against 52.2, 16 -> 32 17.4 against 18.4, 32 -> 32 20.0 against 20.5);
+// with many, or with COUT 96, the weights leave room for one or two CTAs and
+// the persistent kernel's second accumulator set hides the epilogue.
 #define HP_CONV(ci, co)                                                                     \
-  {ci, co, ConvCfg<ci, co>::SMEM, conv3_tc_kernel<ci, co>, RowsCfg<ci, co, CONV_ROWS>::SMEM, \
-   conv3_tc_rows_kernel<ci, co, CONV_ROWS>, 0, nullptr, 0, 0}
+  {ci, co, ALine<ci>::CH, ConvCfg<ci, co>::SMEM, conv3_tc_kernel<ci, co>,                   \
+   RowsCfg<ci, co, CONV_ROWS>::SMEM, conv3_tc_rows_kernel<ci, co, CONV_ROWS>, 0, nullptr, 0, 0}
 #define HP_CONV_P(ci, co)                                                                   \
-  {ci, co, ConvCfg<ci, co>::SMEM, conv3_tc_kernel<ci, co>, RowsCfg<ci, co, CONV_ROWS>::SMEM, \
-   conv3_tc_rows_kernel<ci, co, CONV_ROWS>, PersistCfg<ci, co, 2>::SMEM,                    \
-   conv3_tc_persist_kernel<ci, co, 2>, 2, PersistCfg<ci, co, 2>::COLS}
+  {ci, co, ALine<ci>::CH, ConvCfg<ci, co>::SMEM, conv3_tc_kernel<ci, co>,                   \
+   RowsCfg<ci, co, CONV_ROWS>::SMEM, conv3_tc_rows_kernel<ci, co, CONV_ROWS>,               \
+   PersistCfg<ci, co, 2>::SMEM, conv3_tc_persist_kernel<ci, co, 2>, 2, PersistCfg<ci, co, 2>::COLS}
 static const ConvEntry kConv[] = {
     HP_CONV(16, 16),   HP_CONV(16, 32),   HP_CONV(32, 16),   HP_CONV(32, 32), HP_CONV(32, 64),
     HP_CONV_P(64, 32), HP_CONV_P(64, 64), HP_CONV(48, 16),   HP_CONV_P(96, 32), HP_CONV(16, 48),
@@ -690,7 +795,10 @@ hp_status conv3_launch(const void* X, const void* Wp, const float* bias, void* Y
     return HP_ERR_INVALID;
   }
   CUtensorMap map;
-  hp_status st = make_line_map(&map, X, D, H, W, cin);
+  hp_status st = make_line_map(&map, X, D, H, W, cin, LINE, e->box_c);
+  if (st != HP_OK) return st;
+  CUtensorMap taps;
+  st = make_tap_map(&taps, Wp, cin, cout);
   if (st != HP_OK) return st;
   static bool attr_set[sizeof(kConv) / sizeof(kConv[0])] = {false};
   static int persist_grid[sizeof(kConv) / sizeof(kConv[0])] = {0};
@@ -719,18 +827,18 @@ hp_status conv3_launch(const void* X, const void* Wp, const float* bias, void* Y
     const int n_tiles = (W / TILE_M) * ((H + e->persist_rows - 1) / e->persist_rows) * D;
     const int grid = std::min(n_tiles, persist_grid[idx]);
     e->persist_fn<<<grid, PERSIST_THREADS, e->persist_smem, s>>>(
-        map, (const __nv_bfloat16*)Wp, bias, Y, (const __nv_bfloat16*)mask, D, H, W, epi, err);
+        map, taps, bias, Y, (const __nv_bfloat16*)mask, D, H, W, epi, err);
     HP_CUDA_TRY(cudaGetLastError());
     return HP_OK;
   }
   // Row-blocked CTAs where their two line stages and two weight slices stay
-  // small enough for several CTAs per SM; the wide layers (64+ input or
-  // output channels with large weight slices) keep one line per CTA, which
-  // measured faster there on B200 (e.g. 96 -> 32: 135 vs 156 us).
+  // small enough for several CTAs per SM; else (32 -> 64) one line per CTA:
+  // 15.3 us at 16 x 14 x 128, as the persistent kernel takes, and 19.5 against
+  // 20.5 at 24 x 20 x 128.
   if (e->rows_smem <= 64 * 1024) {
     dim3 grid(W / TILE_M, (H + CONV_ROWS - 1) / CONV_ROWS, D);
-    e->rows_fn<<<grid, 128, e->rows_smem, s>>>(map, (const __nv_bfloat16*)Wp, bias, Y,
-                                               (const __nv_bfloat16*)mask, D, H, W, epi, err);
+    e->rows_fn<<<grid, 128, e->rows_smem, s>>>(map, taps, bias, Y, (const __nv_bfloat16*)mask, D,
+                                               H, W, epi, err);
   } else {
     dim3 grid(W / TILE_M, H, D);
     e->fn<<<grid, 128, e->smem, s>>>(map, (const __nv_bfloat16*)Wp, bias, Y,
@@ -791,7 +899,7 @@ wgrad3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   __shared__ __align__(8) uint64_t done;
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int dz = (int)blockIdx.y - 1;
   const int nl = D * H * WT;
   const int l0 = blockIdx.x * lines_per_cta;
@@ -818,10 +926,11 @@ wgrad3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
   const int nmine = max(0, l1 - l0);
 
-  if (tid == 0 && nmine > 0) {
+  if (warp == 0) {
+    // the warp stays converged; one elected lane issues copies and products
     auto issue = [&](int li, int buf) {
       const int wt = li % WT, h = (li / WT) % H, d = li / (WT * H);
       uint8_t* A = smem + buf * C::STAGE;
@@ -837,53 +946,57 @@ wgrad3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       for (int g = 0; g < N / 8; ++g)
         tma_load_4d(B + g * TILE_M * 16, &tmG, g * 8, wt * TILE_M, h, d, &full[buf]);
     };
-    int issued = 0, consumed = 0;
-    issue(l0, 0);
-    issued = 1;
-    if (nmine > 1) {
-      issue(l0 + 1, 1);
-      issued = 2;
+    int issued = min(nmine, 2), consumed = 0, code = 0;
+    if (elect_one()) {
+      for (int s = 0; s < issued; ++s) issue(l0 + s, s);
     }
+    __syncwarp();
     for (int s = 0; s < nmine; ++s) {
       const int buf = s & 1;
       const uint32_t par = (s >> 1) & 1;
-      if (!mbar_wait(&full[buf], par)) {
-        atomicOr(err, 8);
-        failed = 1;
+      if (!mbar_wait_warp(&full[buf], par)) {
+        code = 8;
         break;
       }
       tc_fence_after();
       const uint32_t a0 = smem_u32(smem + buf * C::STAGE);
-      const uint32_t b0 = a0 + C::A_BYTES;
+      const uint64_t a_d = smem_desc(a0, 128, CHUNK);
+      const uint64_t b_d = smem_desc(a0 + C::A_BYTES, 128, TILE_M * 16);
+      if (elect_one()) {
 #pragma unroll
-      for (int t = 0; t < C::T; ++t) {
+        for (int t = 0; t < C::T; ++t)
 #pragma unroll
-        for (int dx = 0; dx < 3; ++dx) {
+          for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-          for (int k = 0; k < TILE_M / 16; ++k) {
-            const uint64_t ad = smem_desc(a0 + 16 * t * CHUNK + dx * 16 + k * 256, 128, CHUNK);
-            const uint64_t bd = smem_desc(b0 + k * 256, 128, TILE_M * 16);
-            mma_bf16(tmem + (uint32_t)((t * 3 + dx) * N), ad, bd, C::IDESC, (s | k) != 0);
-          }
-        }
+            for (int k = 0; k < TILE_M / 16; ++k)
+              mma_bf16(tmem + (uint32_t)((t * 3 + dx) * N),
+                       desc_add(a_d, 16 * t * CHUNK + dx * 16 + k * 256), desc_add(b_d, k * 256),
+                       C::IDESC, (s | k) != 0);
+        mma_commit(&empty[buf]);
       }
-      mma_commit(&empty[buf]);
+      __syncwarp();
       consumed = s + 1;
       if (s + 2 < nmine) {
-        if (!mbar_wait(&empty[buf], par)) {
-          atomicOr(err, 16);
-          failed = 1;
+        if (!mbar_wait_warp(&empty[buf], par)) {
+          code = 16;
           break;
         }
-        issue(l0 + s + 2, buf);
+        if (elect_one()) issue(l0 + s + 2, buf);
+        __syncwarp();
         ++issued;
       }
     }
-    if (failed) {
-      for (int s = consumed; s < issued; ++s) (void)mbar_wait(&full[s & 1], (s >> 1) & 1);
+    if (code) {
+      for (int s = consumed; s < issued; ++s) (void)mbar_wait_warp(&full[s & 1], (s >> 1) & 1);
+    }
+    if (elect_one()) {
+      if (code) {
+        atomicOr(err, code);
+        failed = 1;
+      }
+      mma_commit(&done);
     }
   }
-  if (tid == 0) mma_commit(&done);
   __syncthreads();
   const bool ok = mbar_wait(&done, 0) && !failed;
   if (!ok && tid == 0) atomicOr(err, 32);

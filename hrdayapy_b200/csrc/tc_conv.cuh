@@ -10,15 +10,16 @@
 //
 // The K loop runs over the 9 (dz, dy) input lines.  For each line a TMA
 // load brings the 130 voxels w0-1 .. w0+128 (zero-filled outside the grid)
-// into shared memory as CIN/8 chunks of [130 voxels][8 channels] -- exactly
-// the no-swizzle K-major core-matrix layout of the UMMA A operand (8 rows of
-// 16 bytes per core matrix, 8-row groups 128 B apart, channel groups one
-// chunk apart).  The three dx taps of the line are the same smem tile with
-// the descriptor start moved by +/-16 bytes (one voxel row), so each line is
-// loaded once and used three times.  The weights of the three taps of the
-// line ([tap][CIN/8][COUT][8], K-major B operand) arrive by one bulk copy.
-// Two smem stages alternate; a single thread issues the TMA copies and the
-// MMAs and commits each stage's MMAs to that stage's "empty" barrier.
+// into shared memory, a voxel's channels as one row of 32, 64 or 128 bytes in
+// the swizzle of that width: a K-major UMMA A operand.  The three dx taps of
+// the line are the same smem tile with the descriptor start moved by +/- one
+// voxel row, so each line is loaded once and used three times.  The weights
+// ([tap][CIN/8][COUT][8], K-major B operand) arrive by bulk copies.  A warp
+// that stays converged walks the stages and one elected lane of it issues the
+// products (under a branch on the thread index the operands of every product
+// are moved to uniform registers one by one, which took about 75 clocks a
+// product, whatever its size), committing each stage's to the stage's "empty"
+// barrier.
 //
 // Every mbarrier wait is bounded: on timeout the CTA records the location in
 // *err, stops issuing work, waits (bounded) for its own copies, frees its
@@ -127,6 +128,15 @@ __device__ __forceinline__ void fence_proxy_async() {
 }
 
 // 4-D tiled TMA load (no multicast), completion on `bar`.
+__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, int c0, int c1,
+                                            int c2, int c3, int c4, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_u32(dst)),
+      "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
+      : "memory");
+}
+
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1,
                                             int c2, int c3, uint64_t* bar) {
   asm volatile(
@@ -159,6 +169,15 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
+// K-major operand whose rows (RB bytes each, 8-row groups 8 RB apart) lie in
+// the swizzle of their width, as TMA writes them; the pattern starts at a
+// multiple of 8 RB (base offset 0) and the leading offset is not used.
+template <int RB>
+__device__ __forceinline__ uint64_t smem_desc_sw(uint32_t saddr) {
+  static_assert(RB == 32 || RB == 64 || RB == 128, "swizzle width");
+  return smem_desc(saddr, 16, 8 * RB) | (uint64_t)(RB == 128 ? 2 : RB == 64 ? 4 : 6) << 61;
+}
+
 // The descriptor of the same layout at saddr + off: the start field holds
 // (address >> 4) in 14 bits and shared-memory addresses stay below 2^18, so
 // adding (off >> 4) never carries into the stride fields.  Lets an MMA loop
@@ -184,6 +203,22 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// True in one lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
+// The whole warp waits; every lane gets the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {

@@ -28,6 +28,7 @@
 #include "precond_apply.cuh"
 
 #include <math.h>
+#include <thread>
 #include <stdint.h>
 
 #include <algorithm>
@@ -384,6 +385,22 @@ static void pcg_kernels(HpTorso* h) {
   h->pcg_fn[1] = h->pairs ? pcg_resident<MODE, true, true> : pcg_resident<MODE, false, true>;
 }
 
+// f(0) .. f(n - 1) on host threads; where one cannot be started, here.  f must
+// not throw.
+template <typename F>
+static void host_parts(int n, F f) {
+  std::vector<std::thread> ts;
+  ts.reserve(n);
+  int t = 1;
+  try {
+    for (; t < n; ++t) ts.emplace_back(f, t);
+  } catch (...) {
+  }
+  for (; t < n; ++t) f(t);
+  f(0);
+  for (auto& x : ts) x.join();
+}
+
 // The resident PCG's tables (pcg_resident.cuh) from the tissue lines, and
 // where a block keeps its vectors: all in shared memory where 36 bytes a pair
 // fit (up to about 1.7 M cells), else r alone (8 bytes, up to about 7.5 M),
@@ -402,60 +419,97 @@ static hp_status setup_pcg(HpTorso* h, const std::vector<int64_t>& line_g0,
   const int n_lines = (int)line_g0.size();
   h->pcg_grid = std::max(1, std::min(nsm, PCG_MAX_BLOCKS));
   std::vector<PcgLine> lines(n_lines);
-  std::vector<uint32_t> meta;
-  std::vector<int64_t> mixed_g;  // first cell of the mixed pairs
   std::vector<int32_t> used(h->pcg_grid, 0);
-  meta.reserve(h->n_rows / 2 + 2 * (int64_t)n_lines);
-  auto cell = [&](int64_t g, int64_t k0, int64_t k1, int64_t k) -> int {
-    return k >= k0 && k < k1 ? lab_u[g] : 0;  // 0: not a cell of the line
-  };
+  int64_t n_pairs = 0;
   for (int l = 0; l < n_lines; ++l) {
     const int64_t row = line_g0[l] / PK, k0 = line_g0[l] % PK, k1 = k0 + line_len[l];
     PcgLine& L = lines[l];
     int32_t& at = used[(l / PCG_WARPS) % h->pcg_grid];  // lines go round by warps
     L.p2 = (uint32_t)(row * PK2 + k0 / 2);
     L.n2 = (int32_t)((k1 + 1) / 2 - k0 / 2);
-    L.c2 = (int32_t)meta.size();
+    L.c2 = (int32_t)n_pairs;
     L.s2 = at;
     L.first = (int32_t)(k0 & 1);
     L.len = line_len[l];
     at += L.n2;
-    for (int64_t k = k0 / 2 * 2; k < k1; k += 2) {
-      const int64_t g = row * PK + k;
-      const int u0 = cell(g, k0, k1, k), u1 = cell(g + 1, k0, k1, k + 1);
+    n_pairs += L.n2;
+  }
+  // The pairs' words and the mixed pairs' coefficients, by host threads over
+  // ranges of lines: mixed pairs are counted within a range first, then moved
+  // by the counts of the ranges before it.
+  struct Part {
+    uint32_t mixed, base;
+    float tu[HP_MAX_MATERIALS], inv[HP_MAX_MATERIALS];
+    bool has[HP_MAX_MATERIALS];
+  };
+  const int n_range = n_lines < 2048
+                         ? 1
+                         : (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+  std::vector<Part> ranges(n_range);
+  std::vector<uint32_t> meta(n_pairs);
+  std::vector<float> mixed;
+  // each pair of the range's lines: f(word, first cell, cells of the pair on the line)
+  auto walk = [&](int t, auto f) {
+    for (int l = (int)((int64_t)n_lines * t / n_range); l < (int64_t)n_lines * (t + 1) / n_range; ++l) {
+      const int64_t row = line_g0[l] / PK, k0 = line_g0[l] % PK, k1 = k0 + line_len[l];
+      uint32_t* m = &meta[lines[l].c2];
+      for (int64_t k = k0 / 2 * 2; k < k1; k += 2, ++m)
+        f(*m, row * PK + k, k >= k0, k + 1 < k1);
+    }
+  };
+  host_parts(n_range, [&](int t) {
+    Part& P = ranges[t];
+    memset(&P, 0, sizeof(P));
+    walk(t, [&](uint32_t& m, int64_t g, bool on0, bool on1) {
+      const int u0 = on0 ? lab_u[g] : 0, u1 = on1 ? lab_u[g + 1] : 0;
       if ((u0 & u1 & LAB_UNIFORM) && !((u0 | u1) & LAB_PIN)) {  // then both are one material
         const int mat = u0 & LAB_MASK;
-        c.tu[mat] = T32[mat * (HP_MAX_MATERIALS + 1)];
-        c.inv[mat] = invd[g];
-        meta.push_back((uint32_t)mat);
+        P.has[mat] = true;
+        P.tu[mat] = T32[mat * (HP_MAX_MATERIALS + 1)];
+        P.inv[mat] = invd[g];
+        m = (uint32_t)mat;
       } else {
-        meta.push_back(PQ_MIXED | (uint32_t)mixed_g.size());
-        mixed_g.push_back(k >= k0 ? g : g | ((int64_t)1 << 62));  // bit 62: the first cell is off the line
-        if (k + 1 >= k1) mixed_g.back() |= (int64_t)1 << 61;      // bit 61: the second is
+        m = PQ_MIXED | P.mixed++;
       }
-    }
+    });
+  });
+  size_t n_mixed = 0;
+  for (Part& P : ranges) {
+    P.base = (uint32_t)n_mixed;
+    n_mixed += P.mixed;
+    for (int mat = 0; mat < HP_MAX_MATERIALS; ++mat)
+      if (P.has[mat]) {
+        c.tu[mat] = P.tu[mat];
+        c.inv[mat] = P.inv[mat];
+      }
   }
+  mixed.resize(14 * n_mixed, 0.0f);
+  host_parts(n_range, [&](int t) {
+    walk(t, [&](uint32_t& m, int64_t g0, bool on0, bool on1) {
+      if (!(m & PQ_MIXED)) return;
+      m += ranges[t].base;
+      const size_t x = m & ~PQ_MIXED;
+      for (int e = 0; e < 2; ++e) {
+        if (!(e ? on1 : on0)) continue;
+        const int64_t g = g0 + e;
+        const int l = lab_u[g] & LAB_MASK;
+        const bool row = l != 0 && !(lab_u[g] & LAB_PIN);
+        for (int f = 0; f < 6 && row; ++f) {
+          const int64_t n = g + nbr[f];
+          float t = T32[l * HP_MAX_MATERIALS + (lab_u[n] & LAB_MASK)];
+          if (!psi.empty()) {
+            const float pa = psi[g], pb = psi[n], sum = pa + pb;
+            t *= sum < 1e-30f ? 0.0f : 2.0f * pa * pb / sum;
+          }
+          mixed[((size_t)f * n_mixed + x) * 2 + e] = t;
+        }
+        mixed[((size_t)6 * n_mixed + x) * 2 + e] = invd[g];
+      }
+    });
+  });
   c.n_lines = n_lines;
   c.n_pairs = (int32_t)meta.size();
-  c.n_mixed = (int32_t)mixed_g.size();
-  std::vector<float> mixed((size_t)14 * mixed_g.size(), 0.0f);
-  for (size_t x = 0; x < mixed_g.size(); ++x)
-    for (int e = 0; e < 2; ++e) {
-      if ((mixed_g[x] >> (62 - e)) & 1) continue;
-      const int64_t g = (mixed_g[x] & (((int64_t)1 << 61) - 1)) + e;
-      const int l = lab_u[g] & LAB_MASK;
-      const bool row = l != 0 && !(lab_u[g] & LAB_PIN);
-      for (int f = 0; f < 6 && row; ++f) {
-        const int64_t n = g + nbr[f];
-        float t = T32[l * HP_MAX_MATERIALS + (lab_u[n] & LAB_MASK)];
-        if (!psi.empty()) {
-          const float pa = psi[g], pb = psi[n], sum = pa + pb;
-          t *= sum < 1e-30f ? 0.0f : 2.0f * pa * pb / sum;
-        }
-        mixed[((size_t)f * mixed_g.size() + x) * 2 + e] = t;
-      }
-      mixed[((size_t)6 * mixed_g.size() + x) * 2 + e] = invd[g];
-    }
+  c.n_mixed = (int32_t)n_mixed;
   c.sj = (uint32_t)PK2;
   c.si = (uint32_t)(PJ * PK2);
   const size_t np = (size_t)(a.ng / PK * PK2) * 2;

@@ -168,7 +168,8 @@ typedef struct HpMono HpMono;
  * returned handle is bound to the current device. */
 hp_status hp_mono_create(const HpMonoDesc *desc, HpMono **out, void *stream);
 /* Advances n steps (n <= remaining).  Kernels are enqueued on `stream`; time
- * loops of `graph_chunk` > 0 steps are replayed from a CUDA graph. */
+ * loops of `graph_chunk` > 0 steps are replayed from a CUDA graph, or, on
+ * hearts that AUTO runs resident, are one cooperative launch. */
 hp_status hp_mono_run(HpMono *h, int64_t n, int32_t graph_chunk, void *stream);
 /* Steps done so far. */
 int64_t hp_mono_steps_done(const HpMono *h);

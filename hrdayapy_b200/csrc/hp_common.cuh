@@ -47,4 +47,19 @@ static hp_status dev_alloc(T** dst, size_t n) {
   return HP_OK;
 }
 
+// Lets launches of a kernel ask for all the dynamic shared memory that its
+// static share leaves.  The limit belongs to the kernel, which the handles of
+// a process share: a handle that set its own size would lower it for a larger
+// handle made before.
+static inline hp_status allow_dynamic_smem(const void* fn) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes at;
+  HP_CUDA_TRY(cudaGetDevice(&dev));
+  HP_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  HP_CUDA_TRY(cudaFuncGetAttributes(&at, fn));
+  HP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   most - (int)at.sharedSizeBytes));
+  return HP_OK;
+}
+
 }  // namespace hp

@@ -1702,8 +1702,7 @@ static hp_status setup_resident(HpMono* h, const HpMonoDesc* d, cudaStream_t s) 
                                   : res_kernel<true, false>(h->res_threads))
                          : (theta ? res_kernel<false, true>(h->res_threads)
                                   : res_kernel<false, false>(h->res_threads));
-  HP_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)h->res_smem));
+  HP_TRY_NODESTROY(allow_dynamic_smem((const void*)fn));
   int fit = 0;
   HP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, (const void*)fn, h->res_threads,
                                                             h->res_smem));

@@ -537,9 +537,7 @@ static hp_status setup_pcg(HpTorso* h, const std::vector<int64_t>& line_g0,
   if (mode == PCG_ALL) pcg_kernels<PCG_ALL>(h);
   else if (mode == PCG_R) pcg_kernels<PCG_R>(h);
   else pcg_kernels<PCG_NONE>(h);
-  for (auto fn : h->pcg_fn)
-    HP_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)h->pcg_smem));
+  for (auto fn : h->pcg_fn) HP_TRY_T(allow_dynamic_smem((const void*)fn));
   if (mode != PCG_ALL) {
     HP_TRY_T(tal(h, &c.Ap, c.n_pairs));
     HP_TRY_T(tal(h, &c.x, c.n_pairs));

@@ -4,7 +4,40 @@ on a kernel may be sized for that handle alone."""
 import numpy as np
 import pytest
 
+from tests.test_pcg_resident_gpu import _box
+
 pytestmark = pytest.mark.gpu
+
+VM = np.array([-80.0, 20.0], np.float32)
+
+
+def _solve(solver):
+    solver.reset()
+    out, st = solver.solve_frame(VM, 1e-4, "rel", 4000)
+    assert st.status == 0 and st.rel_residual <= 1e-4
+    return out
+
+
+@pytest.mark.parametrize("order", [(0, 1), (1, 0)])
+@pytest.mark.parametrize("shapes", [((96, 80, 128), (40, 34, 44)), ((96, 80, 127), (40, 34, 43)),
+                                    ((150, 140, 150), (125, 121, 130))])
+def test_torso_handles_of_two_sizes(shapes, order):
+    """Blocks that keep all vectors on the chip (even and odd padded rows), and
+    the residual alone."""
+    alone = []
+    for shape in shapes:
+        solver, *_ = _box(shape, seed=3)
+        alone.append(_solve(solver))
+        solver.close()
+    both = {}
+    try:
+        for q in order:
+            both[q], *_ = _box(shapes[q], seed=3)
+        for q in (0, 1):
+            np.testing.assert_array_equal(_solve(both[q]), alone[q])
+    finally:
+        for solver in both.values():
+            solver.close()
 
 
 def _heart(shape, theta):

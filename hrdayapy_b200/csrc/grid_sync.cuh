@@ -46,8 +46,13 @@ __device__ __forceinline__ bool grid_sync(const GridSync& g, unsigned long long&
   return s_ok;  // rewritten only after the next barrier's first __syncthreads
 }
 
-// One thread of a block, at the end of the launch: true in the last block out.
+// All threads of a block, at the end of the launch: true in one thread of the
+// last block out.  A block counts as out once every warp of it is here, so
+// what the last one then writes (the counters here, a step count) has been
+// read by all threads of the launch, also where it passed no barrier.
 __device__ __forceinline__ bool grid_last_out(const GridSync& g, unsigned long long epoch) {
+  __syncthreads();
+  if (threadIdx.x != 0) return false;
   __threadfence();
   if (atomicAdd(g.ticket, 1u) != gridDim.x - 1) return false;
   *g.ticket = 0u;

@@ -464,16 +464,13 @@ mono_resident_kernel(MonoArgs a, CnArgs cn, ResArgs rs, int n) {
 #pragma unroll
     for (int v = 0; v < N_STATE; ++v) a.pk_state[(int64_t)v * a.n_pk + p] = cs.v[v];
   }
-  if (threadIdx.x == 0) {
-    if (THETA && blockIdx.x == 0) {
-      cn.iscal[CI_TOTAL] += total;
-      cn.iscal[CI_SOLVES] += n;
-      cn.iscal[CI_UNCONV] += unconv;
-      cn.iscal[CI_BREAK] += breaks;
-    }
-    // the last block out advances the step and barrier counts (all have read them by then)
-    if (grid_last_out(rs.sync, epoch)) *(int64_t*)a.d_step = step0 + n;
+  if (THETA && blockIdx.x == 0 && threadIdx.x == 0) {
+    cn.iscal[CI_TOTAL] += total;
+    cn.iscal[CI_SOLVES] += n;
+    cn.iscal[CI_UNCONV] += unconv;
+    cn.iscal[CI_BREAK] += breaks;
   }
+  if (grid_last_out(rs.sync, epoch)) *(int64_t*)a.d_step = step0 + n;
 }
 
 }  // namespace hp

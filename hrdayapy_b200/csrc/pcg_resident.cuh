@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
       a.x[g + k] = alpha_prev != 0.0 ? x[k] + alpha_prev * (double)p[k] : x[k];
     }
   }
-  if (tid == 0 && grid_last_out(c.sync, epoch)) {
+  if (grid_last_out(c.sync, epoch)) {
     a.scal[SC_RZ] = rz;
     a.scal[SC_PAP] = pAp;
     a.scal[SC_ALPHA] = alpha;

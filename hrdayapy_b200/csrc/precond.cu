@@ -822,10 +822,12 @@ static hp_status coarse_setup(HpPrecond* h, const HpPrecondDesc* d, cudaStream_t
   HP_TRY_PC(pal(h, &h->zc, nc));
   HP_TRY_PC(pal(h, &h->zbox, box2c.size()));
   HP_CUDA_TRY(cudaMemsetAsync(h->zbox, 0, box2c.size() * 4, s));
-  h->seg_len = std::min(ag, 32);
-  h->n_seg = (nk + h->seg_len - 1) / h->seg_len;
-  HP_TRY_PC(pal(h, &h->seg, (size_t)ni * nj * h->n_seg));
-  HP_CUDA_TRY(cudaMemsetAsync(h->seg, 0, (size_t)ni * nj * h->n_seg * 8, s));
+  if (ag >= SEG_MIN) {
+    h->seg_len = std::min(ag, 32);
+    h->n_seg = (nk + h->seg_len - 1) / h->seg_len;
+    HP_TRY_PC(pal(h, &h->seg, (size_t)ni * nj * h->n_seg));
+    HP_CUDA_TRY(cudaMemsetAsync(h->seg, 0, (size_t)ni * nj * h->n_seg * 8, s));
+  }
   HP_CUDA_TRY(cudaMemcpyAsync(h->c_box, c_box.data(), nc * 4, cudaMemcpyHostToDevice, s));
   HP_CUDA_TRY(cudaMemcpyAsync(h->box2c, box2c.data(), box2c.size() * 4, cudaMemcpyHostToDevice, s));
   HP_CUDA_TRY(cudaMemcpyAsync(h->ainv, a32.data(), a32.size() * 4, cudaMemcpyHostToDevice, s));
@@ -1005,6 +1007,7 @@ extern "C" hp_status hp_precond_create(const HpPrecondDesc* d, HpPrecond** out, 
   }
   h->nc = 0;
   h->seg = nullptr;
+  h->seg_len = h->n_seg = 0;
   h->zbox = nullptr;
   if (d->coarse_agg >= 0) PC_TRY(coarse_setup(h, d, s));
   PC_TRY(repack(h, s));
@@ -1095,7 +1098,7 @@ hp_status precond_forward(HpPrecond* h, const uint8_t* label, const float* invd,
 uint64_t precond_serial(const HpPrecond* h) { return h->serial; }
 
 SegArgs precond_segments(const HpPrecond* h) {
-  return SegArgs{h->nc > 0 ? h->seg : nullptr, h->seg_len, h->n_seg, h->nj};
+  return SegArgs{h->seg, h->seg_len, h->n_seg, h->nj};
 }
 
 ZArgs precond_z(const HpPrecond* h, int use_net) {
@@ -1106,7 +1109,10 @@ ZArgs precond_z(const HpPrecond* h, int use_net) {
 
 hp_status precond_update(HpPrecond* h, const uint8_t* label, const float* invd, const float* r,
                          int use_net, cudaStream_t s) {
-  if (h->nc > 0) {
+  if (h->nc > 0 && !h->seg) {
+    const hp_status st = coarse_solve(h, label, r, s);
+    if (st != HP_OK) return st;
+  } else if (h->nc > 0) {
     const CoarseArgs c = coarse_args(h, label);
     const int grid = (h->nc + TB / 32 - 1) / (TB / 32);
     coarse_sum_kernel<<<grid, TB, 0, s>>>(c, precond_segments(h));

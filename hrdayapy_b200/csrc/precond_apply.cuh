@@ -34,7 +34,11 @@ __device__ __forceinline__ float z_value(const ZArgs& z, float inv, float r, int
 }
 
 // Segments of the r update: seg[(i nj + j) n_seg + k / len] is the sum of r
-// over len consecutive cells of a line; null without a coarse level.
+// over len consecutive cells of a line.  Null without a coarse level, and for
+// aggregates of an edge below SEG_MIN: the r update sums four lanes before it
+// looks at len, and the sums would take as many bytes as r itself.  There r is
+// summed per aggregate by a pass of its own.
+constexpr int SEG_MIN = 4;
 struct SegArgs {
   double* seg;
   int len, n_seg, nj;
@@ -42,7 +46,8 @@ struct SegArgs {
 
 SegArgs precond_segments(const HpPrecond* h);
 ZArgs precond_z(const HpPrecond* h, int use_net);
-// zbox = A_c^-1 Q^T r from the segment sums, then the network on r (use_net).
+// zbox = A_c^-1 Q^T r from the segment sums (from r where there are none), then
+// the network on r (use_net).
 hp_status precond_update(HpPrecond* h, const uint8_t* label, const float* invd, const float* r,
                          int use_net, cudaStream_t s);
 // The same from r itself (a residual that no r update has summed).

@@ -237,8 +237,11 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
   double stat = a.scal[SC_STAT], zz = 0.0, rr = 0.0, zmax = 0.0;
   int it = a.iscal[IS_ITER], breakdown = 0, nonfinite = 0;
   for (bool done = false; !done;) {
-    // x += alpha p (the last iteration's step), p = D^-1 r + beta p
+    // x += alpha p (the last iteration's step), p = D^-1 r + beta p.  A
+    // recursion starts with beta = 0 and forgets p, which may hold what a
+    // non-finite solve left (0 * NaN is NaN).
     const float betaf = (float)beta;
+    const bool start = betaf == 0.0f;
     for (int j = 0; j < nl; ++j) {
       const PcgLine L = sl[j * PCG_WARPS];
       double2* x = xs(L);
@@ -255,6 +258,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
           u.y += alpha_prev * (double)pq.y;
           x[q] = u;
         }
+        if (start) pq = make_float2(0.0f, 0.0f);
         pq.x = __fmaf_rn(betaf, pq.x, __fmul_rn(inv.x, rq.x));
         pq.y = __fmaf_rn(betaf, pq.y, __fmul_rn(inv.y, rq.y));
         p[q] = pq;

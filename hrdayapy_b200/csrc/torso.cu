@@ -1152,7 +1152,8 @@ __global__ void __launch_bounds__(TB) fcg_beta(TorsoArgs a, pc::ZArgs z) {
     a.scal[SC_BETA] = -tot[0] / a.scal[SC_PAP];
 }
 
-// p = z + beta p, z = M(r) formed on the fly again
+// p = z + beta p, z = M(r) formed on the fly again; `first` starts a recursion
+// without reading p, which may hold what a non-finite solve left
 __global__ void __launch_bounds__(TB) fcg_p(TorsoArgs a, pc::ZArgs z, int first) {
   if (a.iscal[IS_DONE]) return;
   const float beta = first ? 0.0f : (float)a.scal[SC_BETA];
@@ -1164,7 +1165,7 @@ __global__ void __launch_bounds__(TB) fcg_p(TorsoArgs a, pc::ZArgs z, int first)
   float pb[LB], rb[LB], ib[LB];
   int64_t gb[LB];
   for_aligned_lines<LB>(
-      a, [&](int u, int64_t g) { pb[u] = p[g]; rb[u] = rv[g]; ib[u] = invd[g]; },
+      a, [&](int u, int64_t g) { pb[u] = first ? 0.0f : p[g]; rb[u] = rv[g]; ib[u] = invd[g]; },
       [&](int u, int64_t g, bool on) { gb[u] = g; if (!on) ib[u] = 0.0f; },
       [&](int i, int j, int k) {
 #pragma unroll

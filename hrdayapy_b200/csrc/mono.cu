@@ -1105,7 +1105,9 @@ __global__ void __launch_bounds__(ION_THREADS, 8) mono_ionic_kernel(MonoArgs a, 
     }
     __syncthreads();
   }
-  const float pend = mode == 2 ? (float)*a.cn_pend : 0.0f;  // the solve's last step
+  // the solve's last step; 0 after a breakdown, whose p may be non-finite (0 *
+  // NaN is NaN) and must not reach the x that was kept
+  const float pend = mode == 2 ? (float)*a.cn_pend : 0.0f;
   const bool odd = step & 1;
   const int64_t istep = mode == 1 ? 0 : step + 1;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1114,7 +1116,9 @@ __global__ void __launch_bounds__(ION_THREADS, 8) mono_ionic_kernel(MonoArgs a, 
     const uint32_t tag = a.tag[slot];
     float Vn;
     if constexpr (mode == 2) {
-      Vn = fminf(fmaxf(a.cn_x[slot] + pend * a.cn_p[slot], -150.0f), 80.0f);
+      float x = a.cn_x[slot];
+      if (pend != 0.0f) x += pend * a.cn_p[slot];
+      Vn = fminf(fmaxf(x, -150.0f), 80.0f);
       voxel_outputs(a, slot, tag, Vn, a.Vpost[slot], step, s_vm_frame, s_anim_frame);
     } else {
       Vn = a.Vpost[slot];
@@ -1136,7 +1140,9 @@ __global__ void __launch_bounds__(ION_THREADS, 8) mono_ionic_kernel(MonoArgs a, 
     if (p >= 0 && p < a.n_pk) {
       float Vn;
       if constexpr (mode == 2) {
-        Vn = fminf(fmaxf(a.cn_x[a.n_slots + p] + pend * a.cn_p[a.n_slots + p], -150.0f), 80.0f);
+        float x = a.cn_x[a.n_slots + p];
+        if (pend != 0.0f) x += pend * a.cn_p[a.n_slots + p];
+        Vn = fminf(fmaxf(x, -150.0f), 80.0f);
         a.pk_Vpost[p] = Vn;
         if (s_anim_frame >= 0) a.pk_frames[s_anim_frame * (int64_t)a.n_pk + p] = Vn;
       } else {

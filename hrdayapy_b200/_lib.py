@@ -74,6 +74,8 @@ def lib():
     L.hp_mono_copy_events.argtypes = [P, P, P, P, P, P]
     L.hp_mono_copy_v.argtypes = [P, P, P, P]
     L.hp_mono_copy_state.argtypes = [P, P, P, P]
+    L.hp_mono_status.argtypes = [P]
+    L.hp_mono_inject_timeout.argtypes = [P]
     L.hp_mono_destroy.argtypes = [P]
     L.hp_mono_kernel_info.argtypes = [P, P, P, P]
     _lib = L

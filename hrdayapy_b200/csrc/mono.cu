@@ -1351,6 +1351,9 @@ struct HpMono {
   ResArgs res_a;
   int res_grid, res_threads;
   size_t res_smem;
+  // pinned: set by a resident launch whose barrier gave up, read by the host
+  // without a copy or a wait
+  volatile int32_t* res_failed;
   int cn_grid;       // persistent grid of the set-up pass
   int cn_pgrid;      // persistent grid of the tiled passes
   int cn_vgrid;      // grid of the vector kernels
@@ -1725,6 +1728,10 @@ static hp_status setup_resident(HpMono* h, const HpMonoDesc* d, cudaStream_t s) 
   HP_TRY_NODESTROY(al(h, &r.part, n_part + GRID_SYNC_WORDS));
   HP_CUDA_TRY(cudaMemsetAsync(r.part, 0, (n_part + GRID_SYNC_WORDS) * sizeof(double), s));
   r.sync = grid_sync_at(r.part + n_part);
+  int32_t* failed = nullptr;
+  HP_CUDA_TRY(cudaMallocHost((void**)&failed, sizeof(int32_t)));
+  *failed = 0;
+  h->res_failed = r.sync.err = failed;
   if (theta) {
     r.cg_n = a.n_slots + a.n_pk;
     HP_TRY_NODESTROY(al(h, &r.cg, (size_t)2 * r.cg_n));
@@ -1736,18 +1743,12 @@ static hp_status setup_resident(HpMono* h, const HpMonoDesc* d, cudaStream_t s) 
   return HP_OK;
 }
 
-// After a synchronising copy on s: did a barrier of a resident launch give up
-// (the state is then unusable)?
-static hp_status res_check(const HpMono* h, const char* what, cudaStream_t s) {
-  if (!h->res) return HP_OK;
-  int32_t err = 0;
-  HP_CUDA_TRY(cudaMemcpyAsync(&err, h->res_a.sync.err, sizeof(err), cudaMemcpyDeviceToHost, s));
-  HP_CUDA_TRY(cudaStreamSynchronize(s));
-  if (err) {
-    hp::set_error("%s: a grid barrier of the resident step kernel timed out", what);
-    return HP_ERR_TIMEOUT;
-  }
-  return HP_OK;
+// Has a barrier of a resident launch given up (the state is then unusable)?
+// Sees the launches that the host has waited for.
+static hp_status res_check(const HpMono* h, const char* what) {
+  if (!h->res || !*h->res_failed) return HP_OK;
+  hp::set_error("%s: a grid barrier of the resident step kernel timed out", what);
+  return HP_ERR_TIMEOUT;
 }
 
 extern "C" hp_status hp_mono_create(const HpMonoDesc* d, HpMono** out, void* stream) {
@@ -1806,6 +1807,7 @@ extern "C" hp_status hp_mono_create(const HpMonoDesc* d, HpMono** out, void* str
   h->cn_graph_steps = 0;
   h->cn_graph_stream = nullptr;
   h->res = nullptr;
+  h->res_failed = nullptr;
   h->anisotropic = d->anisotropic;
   h->n_steps = d->n_steps;
   h->steps_done = 0;
@@ -1971,6 +1973,7 @@ extern "C" hp_status hp_mono_run(HpMono* h, int64_t n, int32_t graph_chunk, void
   HP_REQUIRE(n >= 0 && h->steps_done + n <= h->n_steps,
              "hp_mono_run: %lld steps requested, %lld remain", (long long)n,
              (long long)(h->n_steps - h->steps_done));
+  HP_TRY_NODESTROY(res_check(h, "hp_mono_run"));
   cudaStream_t s = (cudaStream_t)stream;
   if (h->res && n >= (h->cn ? 1 : RES_MIN_STEPS)) {
     for (int64_t left = n; left > 0;) {
@@ -2068,7 +2071,7 @@ extern "C" hp_status hp_mono_copy_vm(HpMono* h, int64_t f0, int64_t nf, float* d
   HP_CUDA_TRY(cudaMemcpyAsync(dst, h->a.vm_snap + f0 * h->a.n_myo, nf * h->a.n_myo * sizeof(float),
                               dst_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                               (cudaStream_t)stream));
-  return HP_OK;
+  return res_check(h, "hp_mono_copy_vm");
 }
 
 extern "C" hp_status hp_mono_copy_frames(HpMono* h, int64_t f0, int64_t nf, float* dst_surf,
@@ -2084,7 +2087,7 @@ extern "C" hp_status hp_mono_copy_frames(HpMono* h, int64_t f0, int64_t nf, floa
   if (dst_pk && h->a.n_pk && nf)
     HP_CUDA_TRY(cudaMemcpyAsync(dst_pk, h->a.pk_frames + f0 * h->a.n_pk,
                                 nf * h->a.n_pk * sizeof(float), k, s));
-  return HP_OK;
+  return res_check(h, "hp_mono_copy_frames");
 }
 
 extern "C" hp_status hp_mono_copy_events(HpMono* h, float* act, int32_t* n_act, float* deact,
@@ -2106,7 +2109,7 @@ extern "C" hp_status hp_mono_copy_events(HpMono* h, float* act, int32_t* n_act, 
                                   cudaMemcpyDeviceToHost, s));
       HP_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    HP_TRY_NODESTROY(res_check(h, "hp_mono_copy_events", s));
+    HP_TRY_NODESTROY(res_check(h, "hp_mono_copy_events"));
     for (int64_t i = 0; i < nm; ++i) {
       const int32_t sl = h->slot_of_node[i];
       if (dn) dn[i] = c[sl];
@@ -2167,7 +2170,7 @@ extern "C" hp_status hp_mono_copy_v(HpMono* h, float* v_myo, float* v_pk, void* 
     HP_CUDA_TRY(cudaMemcpyAsync(v.data(), h->a.Vpost, v.size() * sizeof(float),
                                 cudaMemcpyDeviceToHost, s));
     HP_CUDA_TRY(cudaStreamSynchronize(s));
-    HP_TRY_NODESTROY(res_check(h, "hp_mono_copy_v", s));
+    HP_TRY_NODESTROY(res_check(h, "hp_mono_copy_v"));
     for (int64_t i = 0; i < h->a.n_myo; ++i) v_myo[i] = v[h->slot_of_node[i]];
   }
   if (v_pk && h->a.n_pk) {
@@ -2175,7 +2178,7 @@ extern "C" hp_status hp_mono_copy_v(HpMono* h, float* v_myo, float* v_pk, void* 
                                 cudaMemcpyDeviceToHost, s));
     HP_CUDA_TRY(cudaStreamSynchronize(s));
   }
-  return HP_OK;
+  return res_check(h, "hp_mono_copy_v");
 }
 
 extern "C" hp_status hp_mono_copy_state(HpMono* h, float* st_slots, float* st_pk, void* stream) {
@@ -2204,7 +2207,7 @@ extern "C" hp_status hp_mono_copy_state(HpMono* h, float* st_slots, float* st_pk
     HP_CUDA_TRY(cudaMemcpyAsync(st_pk, h->a.pk_state, (size_t)N_STATE * h->a.n_pk * sizeof(float),
                                 cudaMemcpyDeviceToHost, s));
   HP_CUDA_TRY(cudaStreamSynchronize(s));
-  return res_check(h, "hp_mono_copy_state", s);
+  return res_check(h, "hp_mono_copy_state");
 }
 
 extern "C" hp_status hp_mono_cn_stats(HpMono* h, int64_t* iterations, int64_t* solves,
@@ -2216,6 +2219,17 @@ extern "C" hp_status hp_mono_cn_stats(HpMono* h, int64_t* iterations, int64_t* s
   if (solves) *solves = v[CI_SOLVES];
   if (unconverged) *unconverged = v[CI_UNCONV];
   if (breakdowns) *breakdowns = v[CI_BREAK];
+  return res_check(h, "hp_mono_cn_stats");
+}
+
+extern "C" hp_status hp_mono_status(const HpMono* h) {
+  HP_REQUIRE(h, "hp_mono_status: null handle");
+  return res_check(h, "hp_mono_status");
+}
+
+extern "C" hp_status hp_mono_inject_timeout(HpMono* h) {
+  HP_REQUIRE(h && h->res, "hp_mono_inject_timeout: the handle has no resident steps");
+  *h->res_failed = 1;
   return HP_OK;
 }
 
@@ -2225,6 +2239,7 @@ extern "C" hp_status hp_mono_destroy(HpMono* h) {
   if (h->cn_graph) cudaGraphExecDestroy(h->cn_graph);
   if (h->cn_body_stream) cudaStreamDestroy(h->cn_body_stream);
   if (h->cn_host) cudaFreeHost(h->cn_host);
+  if (h->res_failed) cudaFreeHost((void*)h->res_failed);
   for (void* p : h->allocs) cudaFree(p);
   delete h;
   return HP_OK;

@@ -291,11 +291,21 @@ class MonoHandle:
 
     def wait_copies(self):
         """Blocks until every copy started by vm_frames_async has landed."""
+        self._drain_copies()
+        self._check_status()
+
+    def _drain_copies(self):
+        import torch
         cs = getattr(self, "_copy_stream", None)
         if cs is not None:
             cs.synchronize()
         elif getattr(self, "_torch_stream", None) is None:
-            self.sync()
+            torch.cuda.synchronize()
+
+    def _check_status(self):
+        """Raises where a launch that has been waited for gave up at a barrier."""
+        if self.h:
+            _lib.check(_lib.lib().hp_mono_status(self.h), "hp_mono_status")
 
     def vm_frames_device(self, dst_ptr: int, f0: int, nf: int):
         _lib.check(_lib.lib().hp_mono_copy_vm(self.h, f0, nf, C.c_void_p(dst_ptr), 1, self.stream),
@@ -339,10 +349,11 @@ class MonoHandle:
     def sync(self):
         import torch
         torch.cuda.synchronize()
+        self._check_status()
 
     def close(self):
         if getattr(self, "h", None):
-            self.wait_copies()   # no copy may read the snapshots once they are freed
+            self._drain_copies()   # no copy may read the snapshots once they are freed
             _lib.lib().hp_mono_destroy(self.h)
             self.h = None
 

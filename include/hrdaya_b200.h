@@ -178,6 +178,15 @@ int64_t hp_mono_steps_done(const HpMono *h);
  * All zero at theta = 0.  Any output may be NULL; synchronises the device. */
 hp_status hp_mono_cn_stats(HpMono *h, int64_t *iterations, int64_t *solves,
                            int64_t *unconverged, int64_t *breakdowns);
+/* HP_OK, or HP_ERR_TIMEOUT once a grid barrier of a resident launch that the
+ * host has waited for gave up: the handle's state and outputs are then not to
+ * be used.  hp_mono_run, hp_mono_cn_stats and the copies below return the same;
+ * after a copy that returns before it has landed (device or pinned
+ * destinations), ask once it has. */
+hp_status hp_mono_status(const HpMono *h);
+/* Marks a handle with resident steps as such a launch does, for tests of the
+ * caller's error handling. */
+hp_status hp_mono_inject_timeout(HpMono *h);
 /* Step kernel in use (HP_MONO_KERNEL_BRICK, _PIPELINED or _SPLIT), its grid size
  * and dynamic shared memory per CTA; any output may be NULL. */
 hp_status hp_mono_kernel_info(const HpMono *h, int32_t *kernel, int32_t *grid, int64_t *smem_bytes);

@@ -119,6 +119,7 @@ def _declare_optional(L):
     L.hp_torso_copy_solution.argtypes = [P, P, P]
     L.hp_torso_copy_rhs.argtypes = [P, P, P]
     L.hp_torso_reset.argtypes = [P]
+    L.hp_torso_inject_timeout.argtypes = [P, C.c_int32]
     L.hp_torso_destroy.argtypes = [P]
     L.hp_torso_residual_noalloc.argtypes = [C.c_int32, C.c_int32, C.c_int32, P, P, C.c_int32,
                                             C.c_double, C.c_int64, P, P, P, P]

@@ -343,6 +343,7 @@ struct HpTorso {
   int pcg_grid;
   size_t pcg_smem;
   void (*pcg_fn[2])(TorsoArgs, PcgArgs);   // [1]: the p99 rule
+  int fail_in;   // launches until one counts as timed out (hp_torso_inject_timeout), or 0
   cudaGraphExec_t fcg_graph[4];   // FCG chunk without the network / net every 1, 2, 4
   // serial number of the preconditioner handle the FCG graphs hold (not its
   // address: a destroyed handle's address can come back for a new one, whose
@@ -632,6 +633,7 @@ extern "C" hp_status hp_torso_create(const HpTorsoDesc* d, HpTorso** out, void* 
   for (int k = 0; k < 4; ++k) h->fcg_graph[k] = nullptr;
   h->fcg_graph_pc = 0;
   h->fcg_graph_stream = nullptr;
+  h->fail_in = 0;
   h->ni = ni; h->nj = nj; h->nk = nk;
   h->n_rows = n_rows;
   h->have_x = false;
@@ -795,6 +797,14 @@ static hp_status run_iterations(HpTorso* h, bool p99, cudaStream_t s) {
   void* args[] = {&h->a, &h->pcg};
   HP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)h->pcg_fn[p99 ? 1 : 0], dim3(h->pcg_grid),
                                           dim3(32 * PCG_WARPS), args, h->pcg_smem, s));
+  if (h->fail_in > 0 && --h->fail_in == 0)
+    HP_CUDA_TRY(cudaMemsetAsync(h->pcg.sync.err, 1, sizeof(int32_t), s));
+  return HP_OK;
+}
+
+extern "C" hp_status hp_torso_inject_timeout(HpTorso* h, int32_t launch) {
+  HP_REQUIRE(h && launch >= 1, "hp_torso_inject_timeout: null handle or launch < 1");
+  h->fail_in = launch;
   return HP_OK;
 }
 
@@ -1380,8 +1390,7 @@ static hp_status pcg_continue(HpTorso* h, int n, cudaStream_t s) {
   HP_CUDA_TRY(cudaMemcpyAsync(a.iscal, is_run, sizeof(is_run), cudaMemcpyHostToDevice, s));
   hp_status st = run_iterations(h, false, s);
   if (st != HP_OK) return st;
-  HP_CUDA_TRY(cudaStreamSynchronize(s));   // the host scalars above are stack temporaries
-  return HP_OK;
+  return read_scalars(h, s);   // waits: the host scalars above are stack temporaries
 }
 }  // namespace hp
 

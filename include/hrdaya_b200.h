@@ -301,6 +301,10 @@ hp_status hp_torso_copy_solution(HpTorso *h, double *x_rows, void *stream);
 hp_status hp_torso_copy_rhs(HpTorso *h, float *b_rows, void *stream);
 /* Forgets the warm start (next frame starts from zero). */
 hp_status hp_torso_reset(HpTorso *h);
+/* Lets the launch-th launch of PCG iterations from now count as one whose grid
+ * barrier gave up (HP_ERR_TIMEOUT, also of every later solve), for tests of the
+ * caller's error handling. */
+hp_status hp_torso_inject_timeout(HpTorso *h, int32_t launch);
 hp_status hp_torso_destroy(HpTorso *h);
 
 /*

@@ -1,6 +1,6 @@
 """A resident launch whose grid barrier gave up leaves the handle failed, and
 every later call says so.  The tests mark the handle as such a launch does
-(hp_mono_inject_timeout): no wait runs out."""
+(hp_mono_inject_timeout, hp_torso_inject_timeout): no wait runs out."""
 import numpy as np
 import pytest
 
@@ -64,3 +64,21 @@ def test_heart_calls_after_a_timeout(call, theta):
         CALLS[call](sim)
     assert sim.steps_done == done
     sim.close()
+
+
+@pytest.mark.parametrize("launch", [1, 2, 3])
+def test_training_stops_after_a_timeout(launch):
+    """The launches of a training frame: the solve (one recursion at this
+    tolerance), then one for each further iterate."""
+    import torch
+    from hrdayapy_b200 import _lib
+    from hrdayapy_b200.ecg.precond import LearnedPreconditioner
+    from tests.test_precond_gpu import _small, _wave_frames
+    solver, grid, labels, table, dx, vox = _small(shape=(16, 24, 256))
+    pc = LearnedPreconditioner(solver, labels, len(table), coarse_agg=8)
+    vm = torch.from_numpy(np.ascontiguousarray(_wave_frames(vox, 3, 1)[1:2])).cuda()
+    _lib.check(_lib.lib().hp_torso_inject_timeout(solver.h, launch), "hp_torso_inject_timeout")
+    with pytest.raises(_lib.HpError, match="timed out"):
+        pc.train(vm, ks=(4, 8), repeats=1, tol_exact=1e-2)
+    pc.close()
+    solver.close()

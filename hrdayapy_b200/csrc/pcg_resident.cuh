@@ -58,8 +58,10 @@ constexpr int PCG_WARPS = 32;               // a block
 constexpr int PCG_MAX_BLOCKS = 160;
 constexpr int PCG_GROUPS = PCG_MAX_BLOCKS * (PCG_WARPS / 8);  // eight-warp groups
 // where a block keeps its vectors: all in shared memory (36 bytes a pair), r
-// alone (8 bytes a pair), none
-constexpr int PCG_ALL = 0, PCG_R = 1, PCG_NONE = 2;
+// alone (8 bytes a pair), none; PCG_MEM: nor its lines' records, for more of
+// them than shared memory holds (24 bytes each, about 1.3 M on 148
+// multiprocessors; nothing else would fit beside them there)
+constexpr int PCG_ALL = 0, PCG_R = 1, PCG_NONE = 2, PCG_MEM = 3;
 __host__ __device__ constexpr int pcg_pair_bytes(int mode) {
   return mode == PCG_ALL ? 36 : (mode == PCG_R ? 8 : 0);
 }
@@ -188,9 +190,12 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
   const size_t room = c.room;
   PcgLine* sl = (PcgLine*)(pcg_smem + room * pcg_pair_bytes(MODE)) + (tid >> 5);
   const int nl = warp < c.n_lines ? (c.n_lines - 1 - warp) / n_warps + 1 : 0;
-  if (lane == 0)
+  if (MODE != PCG_MEM && lane == 0)
     for (int j = 0; j < nl; ++j) sl[j * PCG_WARPS] = c.line[warp + j * n_warps];
   __syncwarp();
+  auto line = [&](int j) {
+    return MODE == PCG_MEM ? c.line[warp + j * n_warps] : sl[j * PCG_WARPS];
+  };
   // a line's vectors: [pair] of x, r, A p and meta
   auto xs = [&](const PcgLine& L) {
     return MODE == PCG_ALL ? (double2*)pcg_smem + L.s2 : c.x + L.c2;
@@ -216,7 +221,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
     return (int64_t)(L.p2 / c.sj) * a.pk + 2 * (L.p2 % c.sj);
   };
   for (int j = 0; j < nl; ++j) {
-    const PcgLine L = sl[j * PCG_WARPS];
+    const PcgLine L = line(j);
     const int64_t g = grid_cell(L);
     double* x = (double*)xs(L);
     float* r = (float*)rs(L);
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
     const float betaf = (float)beta;
     const bool start = betaf == 0.0f;
     for (int j = 0; j < nl; ++j) {
-      const PcgLine L = sl[j * PCG_WARPS];
+      const PcgLine L = line(j);
       double2* x = xs(L);
       const float2* r = rs(L);
       const uint32_t* m = ms(L);
@@ -269,7 +274,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
     // A p and p.Ap
     double s1[1] = {0.0};
     for (int j = 0; j < nl; ++j) {
-      const PcgLine L = sl[j * PCG_WARPS];
+      const PcgLine L = line(j);
       float2* Ap = As(L);
       const uint32_t* m = ms(L);
       const float2* p = c.p + L.p2;
@@ -340,7 +345,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
     double v[4] = {0.0, 0.0, P99 ? -INFINITY : 0.0, -INFINITY};
     float m2 = -INFINITY, m3 = -INFINITY;
     for (int j = 0; j < nl; ++j) {
-      const PcgLine L = sl[j * PCG_WARPS];
+      const PcgLine L = line(j);
       float* r = (float*)rs(L);
       const float* Ap = (const float*)As(L);
       const uint32_t* m = ms(L);
@@ -410,7 +415,7 @@ __global__ void __launch_bounds__(32 * PCG_WARPS, 1) pcg_resident(TorsoArgs a, P
   }
   // the last step's x, and the vectors back to the padded grid
   for (int j = 0; j < nl; ++j) {
-    const PcgLine L = sl[j * PCG_WARPS];
+    const PcgLine L = line(j);
     const int64_t g = grid_cell(L);
     const double* x = (const double*)xs(L);
     const float* r = (const float*)rs(L);

@@ -405,7 +405,7 @@ static void host_parts(int n, F f) {
 // The resident PCG's tables (pcg_resident.cuh) from the tissue lines, and
 // where a block keeps its vectors: all in shared memory where 36 bytes a pair
 // fit (up to about 1.7 M cells), else r alone (8 bytes, up to about 7.5 M),
-// else none.
+// else none; the lines' records too stay in memory from about 1.3 M on.
 static hp_status setup_pcg(HpTorso* h, const std::vector<int64_t>& line_g0,
                            const std::vector<int32_t>& line_len, const std::vector<uint8_t>& lab_u,
                            const std::vector<float>& psi, const std::vector<float>& invd,
@@ -523,27 +523,30 @@ static hp_status setup_pcg(HpTorso* h, const std::vector<int64_t>& line_g0,
   int dev = 0, most = 0;
   HP_CUDA_TRY(cudaGetDevice(&dev));
   HP_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const size_t line_bytes =
+  const size_t all_lines =
       (size_t)(n_lines + PCG_WARPS * h->pcg_grid - 1) / (PCG_WARPS * h->pcg_grid) * PCG_WARPS *
       sizeof(PcgLine);
-  const size_t taken = 14 * 1024 + line_bytes;  // the reductions' static share, the lines
-  HP_REQUIRE(taken <= (size_t)most, "hp_torso_create: too many tissue lines (%d)", n_lines);
-  const size_t room = (size_t)most - taken;
+  const size_t fixed = 14 * 1024;  // the reductions' static share
+  const bool lines_fit = fixed + all_lines <= (size_t)most;
+  const size_t line_bytes = lines_fit ? all_lines : 0;
+  const size_t room = (size_t)most - fixed - line_bytes;
   const size_t per = ((size_t)*std::max_element(used.begin(), used.end()) + 3) / 4 * 4;
-  const int mode = per * pcg_pair_bytes(PCG_ALL) <= room ? PCG_ALL
-                   : per * pcg_pair_bytes(PCG_R) <= room ? PCG_R
-                                                         : PCG_NONE;
-  c.room = mode == PCG_NONE ? 0 : (int32_t)per;
+  const int mode = !lines_fit                              ? PCG_MEM
+                   : per * pcg_pair_bytes(PCG_ALL) <= room ? PCG_ALL
+                   : per * pcg_pair_bytes(PCG_R) <= room   ? PCG_R
+                                                           : PCG_NONE;
+  c.room = mode == PCG_ALL || mode == PCG_R ? (int32_t)per : 0;
   h->pcg_smem = per * pcg_pair_bytes(mode) + line_bytes;
   if (mode == PCG_ALL) pcg_kernels<PCG_ALL>(h);
   else if (mode == PCG_R) pcg_kernels<PCG_R>(h);
-  else pcg_kernels<PCG_NONE>(h);
+  else if (mode == PCG_NONE) pcg_kernels<PCG_NONE>(h);
+  else pcg_kernels<PCG_MEM>(h);
   for (auto fn : h->pcg_fn) HP_TRY_T(allow_dynamic_smem((const void*)fn));
   if (mode != PCG_ALL) {
     HP_TRY_T(tal(h, &c.Ap, c.n_pairs));
     HP_TRY_T(tal(h, &c.x, c.n_pairs));
   }
-  if (mode == PCG_NONE) HP_TRY_T(tal(h, &c.r, c.n_pairs));
+  if (mode == PCG_NONE || mode == PCG_MEM) HP_TRY_T(tal(h, &c.r, c.n_pairs));
   const size_t n_part = (size_t)2 * PCG_GROUPS * 4;
   HP_TRY_T(tal(h, &c.part, n_part + GRID_SYNC_WORDS));
   HP_CUDA_TRY(cudaMemsetAsync(c.part, 0, (n_part + GRID_SYNC_WORDS) * sizeof(double), s));

@@ -575,7 +575,8 @@ def run_ours(args):
             "config": {"workload": args.workload, "n_voxels": int(n_vox),
                        "n_purkinje": int(prob.n_pk), "dt_ms": prob.dt,
                        "time_steps_per_bench_step": fs, "brick": list(prob.layout.brick),
-                       "kernel": {1: "brick", 2: "pipelined", 3: "split"}[kinfo[0]], "grid": kinfo[1],
+                       "kernel": {1: "brick", 2: "pipelined", 3: "split", 4: "resident"}[kinfo[0]],
+                       "grid": kinfo[1],
                        "autotuned": tune_table is not None,
                        "l2": "working set > L2 (no flush)", "parallelism": f"replicas x{world}"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -583,7 +584,8 @@ def run_ours(args):
                          "traffic_note": traffic_note,
                          "bytes_per_voxel_step": bpv, "peak_source": peak_kind},
             "e2e": e2e,
-            "gpu_launches": int(args.steps * fs * (2 if kinfo[0] == 3 else 1) + args.steps),
+            "gpu_launches": (-(-args.steps * fs // 65536) if kinfo[0] == 4 else
+                             int(args.steps * fs * (2 if kinfo[0] == 3 else 1) + args.steps)),
             "clocks": clk.summary(),
             "check": {"vm_finite": bool(np.isfinite(vm_last).all()),
                       "vm_range_mV": [float(vm_last.min()), float(vm_last.max())]},

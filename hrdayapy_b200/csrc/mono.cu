@@ -2051,6 +2051,12 @@ extern "C" int64_t hp_mono_steps_done(const HpMono* h) { return h ? h->steps_don
 extern "C" hp_status hp_mono_kernel_info(const HpMono* h, int32_t* kernel, int32_t* grid,
                                          int64_t* smem_bytes) {
   HP_REQUIRE(h, "hp_mono_kernel_info: null handle");
+  if (h->res) {
+    if (kernel) *kernel = HP_MONO_KERNEL_RESIDENT;
+    if (grid) *grid = h->res_grid;
+    if (smem_bytes) *smem_bytes = (int64_t)h->res_smem;
+    return HP_OK;
+  }
   if (kernel)
     *kernel = h->diff ? HP_MONO_KERNEL_SPLIT
                       : (h->pipe ? HP_MONO_KERNEL_PIPELINED : HP_MONO_KERNEL_BRICK);

@@ -160,6 +160,7 @@ typedef struct {
 #define HP_MONO_KERNEL_BRICK 1     /* one CTA per brick, plain halo loads */
 #define HP_MONO_KERNEL_PIPELINED 2 /* persistent CTAs, cp.async double-buffered bricks */
 #define HP_MONO_KERNEL_SPLIT 3     /* diffusion launch per brick + ionic launch per tissue slot */
+#define HP_MONO_KERNEL_RESIDENT 4  /* reported only: AUTO on a heart that fits on the chip */
 
 typedef struct HpMono HpMono;
 
@@ -187,8 +188,9 @@ hp_status hp_mono_status(const HpMono *h);
 /* Marks a handle with resident steps as such a launch does, for tests of the
  * caller's error handling. */
 hp_status hp_mono_inject_timeout(HpMono *h);
-/* Step kernel in use (HP_MONO_KERNEL_BRICK, _PIPELINED or _SPLIT), its grid size
- * and dynamic shared memory per CTA; any output may be NULL. */
+/* Step kernel in use (HP_MONO_KERNEL_BRICK, _PIPELINED, _SPLIT or _RESIDENT; a
+ * resident heart's explicit runs of one to three steps take the split kernels),
+ * its grid size and dynamic shared memory per CTA; any output may be NULL. */
 hp_status hp_mono_kernel_info(const HpMono *h, int32_t *kernel, int32_t *grid, int64_t *smem_bytes);
 /* Copies snapshots [f0, f0 + nf) (each n_myo floats, reference node order)
  * to dst; dst_on_device selects cudaMemcpyDeviceToDevice. */

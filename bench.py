@@ -271,7 +271,7 @@ def run_ensemble(args):
                        "variants_per_rank": [r["variants"] for r in per_rank],
                        "parallelism": f"variants sharded over {world} rank(s), LPT",
                        "n_purkinje": int(ens.problem.n_pk), "brick": list(brick),
-                       "kernel": {1: "brick", 2: "pipelined", 3: "split"}[kernel],
+                       "kernel": {0: "auto", 1: "brick", 2: "pipelined", 3: "split"}[kernel],
                        "time_steps_per_bench_step": fs},
             "sequential": {"value": n_vox * steps / (ms_seq * 1e-3),
                            "ms_per_step": ms_seq / args.steps,

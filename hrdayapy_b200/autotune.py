@@ -1,6 +1,7 @@
 """Autotuner for the monodomain step: picks the brick shape and step kernel
-(per-brick, pipelined or split) by timing each candidate on the problem
-itself.
+(AUTO, pipelined or per-brick) by timing each candidate on the problem itself.
+AUTO is the resident steps where the heart fits on the chip and the split step
+elsewhere.
 
 Brick shape decides how many padding slots partially filled bricks carry,
 how large the halo of a tile is and how many CTAs fit an SM; which wins
@@ -25,7 +26,7 @@ from .layout import build_layout
 from .monodomain import MonoProblem
 
 SHAPES = [(4, 4, 8), (4, 8, 8), (2, 4, 16), (8, 8, 8)]
-KERNELS = {1: "brick", 2: "pipelined", 3: "split"}
+KERNELS = {0: "auto", 1: "brick", 2: "pipelined", 3: "split"}
 
 
 def relayout(prob: MonoProblem, brick) -> MonoProblem:
@@ -77,12 +78,13 @@ def _site_on(site_on, n):
     return np.ascontiguousarray(np.stack([np.resize(r, n + 1) for r in a]))
 
 
-def _signature(prob, device_name):
-    return (f"{device_name}|n={prob.n_myo}|pk={prob.n_pk}|aniso={int(prob.anisotropic)}|"
+def _signature(prob, device_name, kernels):
+    return (f"{device_name}|kernels={','.join(map(str, kernels))}|n={prob.n_myo}|pk={prob.n_pk}|"
+            f"aniso={int(prob.anisotropic)}|"
             f"bricks448={prob.layout.n_bricks if tuple(prob.layout.brick) == (4, 4, 8) else -1}")
 
 
-def tune(prob: MonoProblem, shapes=SHAPES, kernels=(3, 2), steps=100, warmup=20,
+def tune(prob: MonoProblem, shapes=SHAPES, kernels=(0, 2), steps=100, warmup=20,
          cache_path=None, verbose=False):
     """Time every (brick shape, kernel) candidate for `steps` steps after
     `warmup` and return (best_problem, table).  table: list of dicts with
@@ -91,7 +93,7 @@ def tune(prob: MonoProblem, shapes=SHAPES, kernels=(3, 2), steps=100, warmup=20,
     import torch
     from . import monodomain as M
     dev = torch.cuda.get_device_name()
-    key = _signature(prob, dev)
+    key = _signature(prob, dev, kernels)
     cache = {}
     if cache_path and Path(cache_path).exists():
         try:

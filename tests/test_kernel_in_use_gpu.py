@@ -54,3 +54,13 @@ def test_resident_is_not_a_kernel_to_ask_for():
     from hrdayapy_b200 import _lib
     with pytest.raises((ValueError, _lib.HpError)):
         _kernel(_slab((8, 8, 8)), RESIDENT)
+
+
+def test_tuned_small_heart_stays_resident():
+    """The resident steps take less than half a split step's time at this size."""
+    from hrdayapy_b200 import monodomain as M
+    from hrdayapy_b200.autotune import tune
+    best, table = tune(_ragged((28, 24, 18)), steps=200, warmup=20)
+    sim = M.MonoHandle(best)
+    assert sim.kernel_info()[0] == RESIDENT, table
+    sim.close()

@@ -1199,13 +1199,14 @@ __global__ void __launch_bounds__(BI * BJ * BK) cn_diag_kernel(MonoArgs a, CnArg
 }
 
 // x += alpha p, r -= alpha q, p = Dinv r + beta p.  In a solve captured in a
-// CUDA graph this ends the body of the conditional WHILE node `loop` (0: none)
+// CUDA graph (in_loop) this ends the body of the conditional WHILE node `loop`
 // and sets whether it runs again: not converged, and fewer than max_iter
 // iterations by its own counter, which bounds the loop whatever the other
 // kernels do.
-__global__ void __launch_bounds__(CN_TB) cn_update_kernel(CnArgs c, cudaGraphConditionalHandle loop) {
+__global__ void __launch_bounds__(CN_TB) cn_update_kernel(CnArgs c, bool in_loop,
+                                                       cudaGraphConditionalHandle loop) {
   const bool done = c.iscal[CI_DONE];
-  if (loop && blockIdx.x == 0 && threadIdx.x == 0) {
+  if (in_loop && blockIdx.x == 0 && threadIdx.x == 0) {
     const int n = ++c.iscal[CI_LOOP];
     cudaGraphSetConditional(loop, (!done && n < c.max_iter) ? 1u : 0u);
   }
@@ -1570,10 +1571,11 @@ static hp_status setup_cn(HpMono* h, const ShapeEntry* se, const HpMonoDesc* d, 
 // One CG iteration of the theta-scheme solve: q = M p (tiled pass: alpha, beta,
 // stopping test), then x, r and p.  Both return at once once the done flag is
 // set.
-static void cn_iteration(HpMono* h, cudaGraphConditionalHandle loop, cudaStream_t s) {
+static void cn_iteration(HpMono* h, const cudaGraphConditionalHandle* loop, cudaStream_t s) {
   const CnArgs& c = h->cn_a;
   h->cn_apply<<<h->cn_pgrid, h->bv, h->diff_smem, s>>>(h->a, c);
-  cn_update_kernel<<<h->cn_vgrid, CN_TB, 0, s>>>(c, loop);
+  cn_update_kernel<<<h->cn_vgrid, CN_TB, 0, s>>>(c, loop != nullptr,
+                                                 loop ? *loop : cudaGraphConditionalHandle{});
 }
 
 // One theta-scheme step: the stencil pass that starts the solve, CG
@@ -1587,7 +1589,7 @@ static hp_status cn_step(HpMono* h, cudaStream_t s) {
   int launched = 0;
   while (launched < c.max_iter) {
     const int k = std::min(h->cn_chunk, c.max_iter - launched);
-    for (int j = 0; j < k; ++j) cn_iteration(h, 0, s);
+    for (int j = 0; j < k; ++j) cn_iteration(h, nullptr, s);
     HP_CUDA_TRY(cudaGetLastError());
     launched += k;
     HP_CUDA_TRY(cudaMemcpyAsync(h->cn_host, c.iscal + CI_DONE, 2 * sizeof(int32_t),
@@ -1629,7 +1631,7 @@ static hp_status cn_capture_steps(HpMono* h, int n, cudaStream_t s) {
     cudaGraph_t body = np.conditional.phGraph_out[0];
     HP_CUDA_TRY(cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0,
                                               cudaStreamCaptureModeRelaxed));
-    cn_iteration(h, hd, sb);
+    cn_iteration(h, &hd, sb);
     cudaGraph_t bo = nullptr;
     HP_CUDA_TRY(cudaStreamEndCapture(sb, &bo));
     HP_CUDA_TRY(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));

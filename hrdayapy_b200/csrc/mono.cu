@@ -2222,7 +2222,11 @@ extern "C" hp_status hp_mono_cn_stats(HpMono* h, int64_t* iterations, int64_t* s
                                       int64_t* unconverged, int64_t* breakdowns) {
   HP_REQUIRE(h, "hp_mono_cn_stats: null handle");
   int32_t v[N_CN_ISCAL] = {0};
-  if (h->cn) HP_CUDA_TRY(cudaMemcpy(v, h->cn_a.iscal, sizeof(v), cudaMemcpyDeviceToHost));
+  if (h->cn) {
+    // a copy on the default stream does not wait for a non-blocking stream's steps
+    HP_CUDA_TRY(cudaDeviceSynchronize());
+    HP_CUDA_TRY(cudaMemcpy(v, h->cn_a.iscal, sizeof(v), cudaMemcpyDeviceToHost));
+  }
   if (iterations) *iterations = v[CI_TOTAL];
   if (solves) *solves = v[CI_SOLVES];
   if (unconverged) *unconverged = v[CI_UNCONV];

@@ -43,3 +43,18 @@ def test_tiled_theta_graph_and_host_loop_agree(cg_max_iter):
     in the same order, also where the iteration limit ends the loop."""
     its, solves, unconverged, _ = _runs(0.5, (0, 1, 16), cg_max_iter)
     assert its <= cg_max_iter * solves and (unconverged > 0) == (cg_max_iter < 100)
+
+
+def test_counters_are_of_all_steps_enqueued():
+    """cn_stats waits for the steps before it."""
+    from hrdayapy_b200 import monodomain as M
+    args, fibre, kw = cases.ragged_aniso_case(T=40.0)
+    nodes, el, act, S, phi = args
+    prob, _ = M.prepare(nodes, el, act, S, S, phi, fibre_dir=fibre, anisotropic=True, theta=0.5,
+                        cg_tol=1e-6, **dict(kw, A_P=2.0 / kw["R_P"]))
+    for kernel in (0, 3):
+        n = prob.n_steps // 16 * 16
+        sim = M.MonoHandle(dataclasses.replace(prob, kernel=kernel))
+        sim.run(n, graph_chunk=16)
+        assert sim.cn_stats()[1] == n
+        sim.close()

@@ -1484,7 +1484,9 @@ extern "C" hp_status hp_torso_copy_rhs(HpTorso* h, float* b_rows, void* stream) 
 
 extern "C" hp_status hp_torso_reset(HpTorso* h) {
   HP_REQUIRE(h, "hp_torso_reset: null handle");
-  HP_CUDA_TRY(cudaMemset(h->a.x, 0, h->a.ng * 8));
+  // in the default stream, which a caller's non-blocking stream does not wait for
+  HP_CUDA_TRY(cudaMemsetAsync(h->a.x, 0, h->a.ng * 8, cudaStreamLegacy));
+  HP_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
   h->have_x = false;
   return HP_OK;
 }

@@ -1260,6 +1260,12 @@ static hp_status fcg_run(HpTorso* h, HpPrecond* p, double tol, int fallback_iter
     *it_out = 0;
     return HP_OK;
   }
+  if (!isfinite(bb) || !isfinite(h->h_scal[SC_TRUE_RR])) {  // rel says nothing; the plain PCG reports it
+    *rel_out = rel;
+    *it_out = 0;
+    *fallback = true;
+    return HP_OK;
+  }
   // chunks of FCG_CHUNK iterations replayed from a CUDA graph; kernels of a
   // chunk after the device-side done flag return at once (the
   // preconditioner's then only writes its own scratch and z)

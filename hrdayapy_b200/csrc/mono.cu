@@ -30,6 +30,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 namespace hp {
@@ -1671,6 +1672,39 @@ static hp_status cn_build_graph(HpMono* h, int n, cudaStream_t s) {
   return HP_OK;
 }
 
+// Words of pinned host memory for the handles' failure flags.  Pinning memory
+// for each handle took 2.8 ms of a small heart's 4.0 ms creation and 0.5 ms of
+// its destruction, so words come from pages of 1,024 that stay pinned and go
+// back to their list with the handle: one page serves all but a process with
+// more resident hearts alive at once.  Portable: any device's launches write them.
+struct FlagWords {
+  std::mutex lock;
+  std::vector<int32_t*> free;
+};
+static FlagWords& flag_words() {
+  static FlagWords* w = new FlagWords;  // outlives every handle
+  return *w;
+}
+static hp_status flag_take(int32_t** out) {
+  constexpr int WORDS = 1024;
+  FlagWords& w = flag_words();
+  std::lock_guard<std::mutex> hold(w.lock);
+  if (w.free.empty()) {
+    int32_t* page = nullptr;
+    HP_CUDA_TRY(cudaHostAlloc((void**)&page, WORDS * sizeof(int32_t), cudaHostAllocPortable));
+    for (int k = 0; k < WORDS; ++k) w.free.push_back(page + k);
+  }
+  *out = w.free.back();
+  w.free.pop_back();
+  **out = 0;
+  return HP_OK;
+}
+static void flag_give(int32_t* word) {
+  FlagWords& w = flag_words();
+  std::lock_guard<std::mutex> hold(w.lock);
+  w.free.push_back(word);
+}
+
 // The register budget per block size: up to 256 threads a block has 128
 // registers and two or more handles' blocks share an SM; up to 448 threads 72
 // registers keep two blocks on an SM (64 x 64 x 16 slab, three handles in
@@ -1730,10 +1764,8 @@ static hp_status setup_resident(HpMono* h, const HpMonoDesc* d, cudaStream_t s) 
   HP_TRY_NODESTROY(al(h, &r.part, n_part + GRID_SYNC_WORDS));
   HP_CUDA_TRY(cudaMemsetAsync(r.part, 0, (n_part + GRID_SYNC_WORDS) * sizeof(double), s));
   r.sync = grid_sync_at(r.part + n_part);
-  int32_t* failed = nullptr;
-  HP_CUDA_TRY(cudaMallocHost((void**)&failed, sizeof(int32_t)));
-  *failed = 0;
-  h->res_failed = r.sync.err = failed;
+  HP_TRY_NODESTROY(flag_take(&r.sync.err));
+  h->res_failed = r.sync.err;
   if (theta) {
     r.cg_n = a.n_slots + a.n_pk;
     HP_TRY_NODESTROY(al(h, &r.cg, (size_t)2 * r.cg_n));
@@ -2251,8 +2283,8 @@ extern "C" hp_status hp_mono_destroy(HpMono* h) {
   if (h->cn_graph) cudaGraphExecDestroy(h->cn_graph);
   if (h->cn_body_stream) cudaStreamDestroy(h->cn_body_stream);
   if (h->cn_host) cudaFreeHost(h->cn_host);
-  if (h->res_failed) cudaFreeHost((void*)h->res_failed);
   for (void* p : h->allocs) cudaFree(p);
+  if (h->res_failed) flag_give((int32_t*)h->res_failed);  // no launch is left that could set it
   delete h;
   return HP_OK;
 }

@@ -82,3 +82,18 @@ def test_training_stops_after_a_timeout(launch):
         pc.train(vm, ks=(4, 8), repeats=1, tol_exact=1e-2)
     pc.close()
     solver.close()
+
+
+def test_a_timeout_is_of_one_handle():
+    """Not of the others alive, nor of the next one made."""
+    from hrdayapy_b200 import _lib
+    a, b = _heart(), _heart(0.5)
+    _lib.check(_lib.lib().hp_mono_inject_timeout(a.h), "hp_mono_inject_timeout")
+    b.run(4)
+    b.vm_frames()
+    a.close()
+    c = _heart()
+    c.run(4)
+    c.vm_frames()
+    b.close()
+    c.close()

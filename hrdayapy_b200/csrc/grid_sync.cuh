@@ -15,7 +15,7 @@ struct GridSync {
   unsigned long long* count;  // arrivals since creation
   unsigned long long* epoch;  // barriers passed since creation
   unsigned int* ticket;       // blocks that are through with the launch
-  int32_t* err;               // set when a barrier ran out of its polls; read back with the results
+  int32_t* err;               // set when a barrier ran out of its polls (device or pinned host memory)
 };
 constexpr int GRID_SYNC_WORDS = 4;  // 8-byte words the four counters take, all zero at first
 
